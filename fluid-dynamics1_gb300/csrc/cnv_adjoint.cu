@@ -224,6 +224,21 @@ void free_adjoint(cnv_adjoint* a) {
     delete a;
 }
 
+// Before a run: no abort of an earlier one left, the solve's barrier armed.
+int begin_run(cnv_adjoint* a) {
+    ACUDA(cudaMemsetAsync(a->ctrl, 0, sizeof(Ctrl), a->stream));
+    ACUDA(dst_reset(a->dst, a->stream));
+    return CNV_OK;
+}
+
+// After a run: waits for it, and reports a solve whose blocks gave up waiting for one another.
+int end_run(cnv_adjoint* a) {
+    Ctrl h{};
+    ACUDA(cudaMemcpyAsync(&h, a->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, a->stream));
+    ACUDA(cudaStreamSynchronize(a->stream));
+    return h.abort ? afail(h.status != CNV_OK ? h.status : CNV_CUDA_ERROR, "grid barrier wait timed out") : CNV_OK;
+}
+
 size_t nn_of(const cnv_adjoint* a) { return (size_t)a->n * a->n; }
 
 double* slot_w(double* base, size_t nn, size_t k) { return base + 3 * nn * k; }
@@ -286,6 +301,8 @@ int run_forward(cnv_adjoint* a, const double* w0_dev, double lid, int nsteps, bo
         int rc = ensure_slots(a->guards, &a->ck, &a->ck_slots, std::max<size_t>(want, 1), nn, "checkpoints");
         if (rc != CNV_OK) return rc;
     }
+    const int rc0 = begin_run(a);
+    if (rc0 != CNV_OK) return rc0;
     ACUDA(cudaMemcpyAsync(a->w[0], w0_dev, nn * 8, cudaMemcpyDeviceToDevice, a->stream));
     ACUDA(cudaMemcpyAsync(a->u, a->u0, nn * 8, cudaMemcpyDeviceToDevice, a->stream));
     ACUDA(cudaMemcpyAsync(a->v, a->v0, nn * 8, cudaMemcpyDeviceToDevice, a->stream));
@@ -313,6 +330,7 @@ int run_backward(cnv_adjoint* a, const double* gT_dev, double* gw0_dev, double* 
     const size_t nn = nn_of(a);
     const int n = a->n;
     int rc = ensure_slots(a->guards, &a->seg, &a->seg_slots, (size_t)a->every + 1, nn, "segment states");
+    if (rc == CNV_OK) rc = begin_run(a);
     if (rc != CNV_OK) return rc;
     ACUDA(cudaEventRecord(a->ev[2], a->stream));
     ACUDA(cudaMemcpyAsync(a->lw, gT_dev, nn * 8, cudaMemcpyDeviceToDevice, a->stream));
@@ -370,7 +388,7 @@ int run_backward(cnv_adjoint* a, const double* gT_dev, double* gw0_dev, double* 
     if (gw0_dev) ACUDA(cudaMemcpyAsync(gw0_dev, a->lw, nn * 8, cudaMemcpyDeviceToDevice, a->stream));
     std::vector<double> row(n);
     ACUDA(cudaMemcpyAsync(row.data(), a->lid_row, n * 8, cudaMemcpyDeviceToHost, a->stream));
-    ACUDA(cudaStreamSynchronize(a->stream));
+    if ((rc = end_run(a)) != CNV_OK) return rc;
     double s = 0;
     for (int j = 1; j < n - 1; ++j) s += row[j];
     if (g_lid) *g_lid = s;
@@ -452,7 +470,7 @@ int cnv_adjoint_create(const cnv_config* cfg, int checkpoint_every, cnv_adjoint*
         return afail(CNV_BAD_ARG, "finite-difference bands");
     }
     if (cudaMemcpy(a->bands, &hb, sizeof hb, cudaMemcpyHostToDevice) != cudaSuccess) return bad("band upload");
-    if (dst_plan_create(n, a->dx, a->dy, &a->dst) != CNV_OK) return bad("sine-transform plan");
+    if (dst_plan_create(n, cfg->Lx, cfg->Ly, a->ctrl, 2000000000LL, &a->dst) != CNV_OK) return bad("sine-transform plan");
     // initial velocities of src/main.c:213-221: ui, vi on the interior, zero on the edges
     std::vector<double> hu(nn, 0.0), hv(nn, 0.0);
     for (int i = 1; i < n - 1; ++i)
@@ -477,7 +495,7 @@ int cnv_adjoint_forward_device(cnv_adjoint* a, const double* w0, double lid, int
     if (rc != CNV_OK) return rc;
     if (w_final)
         ACUDA(cudaMemcpyAsync(w_final, a->w[a->cur], nn_of(a) * 8, cudaMemcpyDeviceToDevice, a->stream));
-    ACUDA(cudaStreamSynchronize(a->stream));
+    if ((rc = end_run(a)) != CNV_OK) return rc;
     float ms = 0;
     cudaEventElapsedTime(&ms, a->ev[0], a->ev[1]);
     a->fwd_ms = ms;
@@ -501,7 +519,7 @@ int cnv_adjoint_forward(cnv_adjoint* a, const double* w0, double lid, int nsteps
     if (rc != CNV_OK) return rc;
     std::vector<double> h(nn);
     ACUDA(cudaMemcpyAsync(h.data(), a->w[a->cur], nn * 8, cudaMemcpyDeviceToHost, a->stream));
-    ACUDA(cudaStreamSynchronize(a->stream));
+    if ((rc = end_run(a)) != CNV_OK) return rc;
     float ms = 0;
     cudaEventElapsedTime(&ms, a->ev[0], a->ev[1]);
     a->fwd_ms = ms;

@@ -265,6 +265,7 @@ int reset_ctrl(cnv_state* s) {
     h.records = s->records;
     h.max_records = s->max_records;
     CNV_CUDA(cudaMemcpyAsync(s->ctrl, &h, sizeof(Ctrl), cudaMemcpyHostToDevice, s->stream));
+    if (s->direct) CNV_CUDA(dst_reset(s->dst, s->stream));
     return CNV_OK;
 }
 
@@ -325,9 +326,7 @@ MixedLaunch mixed_launch(cnv_state* s) {
 // (w with c4 in a step, f with -c4 for a standalone solve) and reports 0 iterations.
 int enqueue_poisson(cnv_state* s, const double* in, double scale, bool in_step) {
     const size_t split_bytes = (size_t)s->n * s->pitch * 8;
-    if (s->direct) {
-        CNV_CUDA(cudaMemsetAsync(s->sor[0], 0, split_bytes, s->stream));
-        CNV_CUDA(cudaMemsetAsync(s->sor[1], 0, split_bytes, s->stream));
+    if (s->direct) {  // it writes the interior alone: the edges keep upload_initial's zeros
         CNV_CUDA(dst_solve_split(s->dst, in, scale, s->sor[0], s->sor[1], s->pitch, s->stream));
         // iters, status (int) and err (double) of the control block: 0, CNV_OK, 0.0
         static_assert(offsetof(Ctrl, status) == offsetof(Ctrl, iters) + 4 && offsetof(Ctrl, err) == offsetof(Ctrl, iters) + 8,
@@ -595,7 +594,8 @@ int cnv_create(const cnv_config* cfg, cnv_state** out) {
     }
     if (cfg->poisson_type == CNV_POISSON_DIRECT) {
         s->direct = true;
-        if (dst_plan_create(n, s->dx, s->dy, &s->dst) != CNV_OK) {
+        if (dst_plan_create(n, cfg->Lx, cfg->Ly, s->ctrl,
+                            (cfg->solver_timeout_ms > 0 ? cfg->solver_timeout_ms : 2000) * 1000000LL, &s->dst) != CNV_OK) {
             free_state(s);
             return fail(CNV_CUDA_ERROR, "sine-transform plan for n = %d", n);
         }
