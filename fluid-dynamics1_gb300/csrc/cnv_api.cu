@@ -122,6 +122,7 @@ struct cnv_state {
     void* msync = nullptr;
     int mixed_gx = 1, mixed_gy = 1, mixed_epochs = 1, mixed_max_outer = 100;
     bool mixed_rq_smem = false;
+    int mixed_form = -1, mixed_ntx = 0, mixed_nty = 0;
     double mixed_rtol = 1e-10;
     // several sweeps per border exchange (FP64 SOR/GS in shared-memory tiles)
     bool tb = false;
@@ -308,6 +309,9 @@ MixedLaunch mixed_launch(cnv_state* s) {
     L.max_outer = s->mixed_max_outer;
     L.epochs = s->mixed_epochs;
     L.rq_in_smem = s->mixed_rq_smem ? 1 : 0;
+    L.form = s->mixed_form;
+    L.ntx = s->mixed_ntx;
+    L.nty = s->mixed_nty;
     L.timeout_ns = s->pp.timeout_ns;
     const size_t split = (size_t)s->n * s->pitch;
     for (int c = 0; c < 2; ++c) {
@@ -316,6 +320,7 @@ MixedLaunch mixed_launch(cnv_state* s) {
         L.rq[c] = s->rq + c * split;
         for (int par = 0; par < 2; ++par) L.eg[par][c] = s->eg + (2 * par + c) * split;
     }
+    L.eg2 = reinterpret_cast<uint2*>(s->eg);
     L.ctrl = s->ctrl;
     L.sync = s->msync;
     return L;
@@ -532,10 +537,20 @@ int cnv_create(const cnv_config* cfg, cnv_state** out) {
         // every tile at least as wide and tall as the halo, so a halo comes from the eight
         // adjacent tiles only
         const int halo = 2 * mixed_sweeps_per_exchange();
-        for (int g = std::min(s->sms, kMaxSolverBlocks); g >= 1; --g) {
+        const auto tiles_ok = [&](int g) {
             poisson_tiles(n, g, &s->mixed_gx, &s->mixed_gy);
-            if ((n - 2) / s->mixed_gx >= halo && (n - 2) / s->mixed_gy >= halo) break;
-            s->mixed_gx = s->mixed_gy = 1;
+            return (n - 2) / s->mixed_gx >= halo && (n - 2) / s->mixed_gy >= halo;
+        };
+        // the most tiles the register kernel takes, else the most that are wide enough for the shared-memory one
+        int g = std::min(s->sms, kMaxSolverBlocks);
+        for (; g >= 1; --g) {
+            if (!tiles_ok(g)) continue;
+            mixed_pick(n, s->mixed_gx, s->mixed_gy, prop.sharedMemPerBlockOptin, &s->mixed_form, &s->mixed_ntx, &s->mixed_nty);
+            if (s->mixed_form >= 0) break;
+        }
+        if (g < 1) {
+            for (g = std::min(s->sms, kMaxSolverBlocks); g >= 1 && !tiles_ok(g);) --g;
+            if (g < 1) s->mixed_gx = s->mixed_gy = 1;
         }
         s->mixed_rq_smem = mixed_smem_bytes(n, s->mixed_gx, s->mixed_gy, true) + 2048 <= prop.sharedMemPerBlockOptin;
         const size_t smem = mixed_smem_bytes(n, s->mixed_gx, s->mixed_gy, s->mixed_rq_smem);
@@ -549,14 +564,15 @@ int cnv_create(const cnv_config* cfg, cnv_state** out) {
         s->mixed_max_outer = cfg->mixed_max_outer > 0 ? cfg->mixed_max_outer : 100;
         s->mixed_rtol = cfg->mixed_rtol > 0 ? cfg->mixed_rtol : 1e-10;
         ALLOC(s->rq, 2 * split);
-        ALLOC(s->eg, 4 * split);
+        const size_t eg_floats = (s->mixed_form >= 0 ? 8 : 4) * split;
+        ALLOC(s->eg, eg_floats);
         cudaError_t e_ = cudaMalloc(&s->msync, mixed_sync_bytes());
         if (e_ != cudaSuccess) {
             free_state(s);
             return fail(CNV_CUDA_ERROR, "cudaMalloc: %s", cudaGetErrorString(e_));
         }
         if (cudaMemsetAsync(s->rq, 0, 2 * split * 4, s->stream) != cudaSuccess ||
-            cudaMemsetAsync(s->eg, 0, 4 * split * 4, s->stream) != cudaSuccess) {
+            cudaMemsetAsync(s->eg, 0, eg_floats * 4, s->stream) != cudaSuccess) {
             free_state(s);
             return fail(CNV_CUDA_ERROR, "initial memset failed");
         }

@@ -83,18 +83,21 @@ struct MixedLaunch {
     int n, pitch, gx, gy;
     double dx2, dy2, den, rden, beta, rtol;
     int max_outer, epochs;
+    int form, ntx, nty;  // register kernel's form and threads across and down its box (form -1: shared-memory tiles)
     int rq_in_smem;   // keep the correction right-hand side tile in shared memory
     long long timeout_ns;
     const double* g[2];
     double* psi[2];
     float* rq[2];
     float* eg[2][2];  // [parity][colour]
+    uint2* eg2;       // the same memory, for the register kernel: [parity][colour] fields of (e, epoch)
     Ctrl* ctrl;
     void* sync;
 };
 cudaError_t launch_mixed(const MixedLaunch& L, cudaStream_t s);
 size_t mixed_sync_bytes();
 size_t mixed_smem_bytes(int n, int gx, int gy, bool rq_in_smem);
+void mixed_pick(int n, int gx, int gy, size_t smem_max, int* form, int* ntx, int* nty);
 int mixed_threads();
 int mixed_sweeps_per_exchange();
 
