@@ -71,8 +71,8 @@ struct DstDest {
 
 // ------------------------------------------------------------------ FFT in shared memory, in FP32 or FP64 (R)
 template <class R> struct Pair;
-template <> struct Pair<float> { typedef float2 t; };
-template <> struct Pair<double> { typedef double2 t; };
+template <> struct Pair<float> { typedef float2 t; typedef double wide; };
+template <> struct Pair<double> { typedef double2 t; typedef long double wide; };
 template <class R> using C2 = typename Pair<R>::t;
 __device__ __forceinline__ float2 c2(float x, float y) { return make_float2(x, y); }
 __device__ __forceinline__ double2 c2(double x, double y) { return make_double2(x, y); }
@@ -1002,6 +1002,28 @@ int solves_needed(int len, int radix, double a2, double b2) {
     return std::max(k, 3);
 }
 
+// exp(2 pi i t / M), M = 4 len, in W: computed for the first eighth of the circle, exact symmetries for the rest (on an Arm
+// host a long double sine takes a microsecond of software).
+template <class W>
+struct Roots {
+    int len;
+    std::vector<W> c, s;
+    explicit Roots(int len) : len(len), c(len / 2 + 1), s(len / 2 + 1) {
+        const W pi = (W)3.141592653589793238462643383279502884L;
+        for (int t = 0; t <= len / 2; ++t) {
+            c[t] = std::cos(pi * t / (2 * len));
+            s[t] = std::sin(pi * t / (2 * len));
+        }
+    }
+    W first(int r, bool sine) const { return 2 * r <= len ? (sine ? s[r] : c[r]) : (sine ? c[len - r] : s[len - r]); }
+    W cos(long long t) const {  // t >= 0
+        const int q = (int)(t / len % 4), r = (int)(t % len);
+        const W v = first(r, q & 1);
+        return q == 1 || q == 2 ? -v : v;
+    }
+    W sin(long long t) const { return cos(t + 3LL * len); }
+};
+
 // The FFT path's tables and fields for len = m + 1; false where it does not apply.
 template <class R>
 bool plan_fft(DstPlan* P, int a, int b, int sms, int smem_max, const Ctrl* ctrl, int* status) {
@@ -1065,34 +1087,27 @@ bool plan_fft(DstPlan* P, int a, int b, int sms, int smem_max, const Ctrl* ctrl,
         L *= S.p;
         off += S.p;
     }
-    // tables in long double, rounded once
-    const long double pi = 3.141592653589793238462643383279502884L;
+    const Roots<typename Pair<R>::wide> roots(len);  // exp(2 pi i t / 4N), from which every table comes
     std::vector<C2<R>> tw(len), cs(ncs), sc(len / 2 + 1);
     std::vector<R> li(len + 1, R(0)), lj(len + 1, R(0));
-    for (int t = 0; t < len; ++t) {
-        const long double x = 2 * pi * t / len;  // exp(-2 pi i t / N)
-        tw[t] = C2<R>{(R)std::cos(x), (R)-std::sin(x)};
-    }
-    for (int t = 0; t <= len / 2; ++t) sc[t] = C2<R>{(R)std::sin(pi * t / len), (R)std::cos(pi * t / len)};
+    for (int t = 0; t < len; ++t) tw[t] = C2<R>{(R)roots.cos(4 * t), (R)-roots.sin(4 * t)};  // exp(-2 pi i t / N)
+    for (int t = 0; t <= len / 2; ++t) sc[t] = C2<R>{(R)roots.sin(2 * t), (R)roots.cos(2 * t)};
     for (int s = 0; s < F.nstages; ++s)
-        for (int t = 0; t < rad[s]; ++t) {
-            const long double x = 2 * pi * t / rad[s];
-            cs[F.st[s].csoff + t] = C2<R>{(R)std::cos(x), (R)std::sin(x)};
-        }
+        for (int t = 0; t < rad[s]; ++t)
+            cs[F.st[s].csoff + t] = C2<R>{(R)roots.cos(4 * t * (len / rad[s])), (R)roots.sin(4 * t * (len / rad[s]))};
     for (int k = 1; k <= m; ++k) {
-        const long double sk = std::sin(pi * k / (2.0L * len));
-        li[k] = (R)(4.0L * (kF64 ? (long double)P->dy2 : F.a2) * sk * sk);
-        lj[k] = (R)(4.0L * (kF64 ? (long double)P->dx2 : F.b2) * sk * sk);
+        const auto sk = roots.sin(k);
+        li[k] = (R)(4 * (kF64 ? P->dy2 : (double)F.a2) * sk * sk);
+        lj[k] = (R)(4 * (kF64 ? P->dx2 : (double)F.b2) * sk * sk);
     }
     std::vector<R> cm(std::max(ncm, 1));
     for (int s = 0; s < F.nstages; ++s) {
         const FftStage& S = F.st[s];
         for (int q = 1; S.pad && q <= (S.p - 1) / 2; ++q)
             for (int k = 0; k < S.pad; ++k) {
-                const long double x = 2 * pi * (q * k % S.p) / S.p;
                 R* row = cm.data() + S.cmoff + 2 * q * S.pad + k;
-                row[0] = (R)std::cos(x);
-                row[S.pad] = (R)std::sin(x);
+                row[0] = cs[S.csoff + q * k % S.p].x;
+                row[S.pad] = cs[S.csoff + q * k % S.p].y;
             }
     }
     // one allocation: tables, then the fields (zeroed: their edges stay zero)
@@ -1112,8 +1127,9 @@ bool plan_fft(DstPlan* P, int a, int b, int sms, int smem_max, const Ctrl* ctrl,
         at += align(part[k]);
     }
     const void* tables[] = {tw.data(), sc.data(), li.data(), lj.data(), cm.data(), cs.data()};
-    for (int k = 0; k < kTables; ++k)
-        if (cudaMemcpy(ptr[k], tables[k], part[k], cudaMemcpyHostToDevice) != cudaSuccess) return true;
+    std::vector<char> host(ptr[kTables] - ptr[0], 0);
+    for (int k = 0; k < kTables; ++k) std::memcpy(host.data() + (ptr[k] - ptr[0]), tables[k], part[k]);
+    if (cudaMemcpy(P->arena, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess) return true;
     F.tables = ptr[0];
     F.off_sc = (int)(ptr[1] - ptr[0]);
     F.off_li = (int)(ptr[2] - ptr[0]);
