@@ -131,6 +131,9 @@ struct cnv_state {
     bool tb_g_smem = false;
     double* tb_snap = nullptr;
     void* tb_sync = nullptr;
+    // FP64 SOR/GS with a cell of each colour per thread (cells.tc > 0)
+    CellsPlan cells{};
+    void* cells_sync = nullptr;
     // exact solve by sine transforms (CNV_POISSON_DIRECT)
     bool direct = false;
     DstPlan dst{};
@@ -184,6 +187,7 @@ void free_state(cnv_state* s) {
     if (s->msync) cudaFree(s->msync);
     buf_free(s, s->tb_snap);
     if (s->tb_sync) cudaFree(s->tb_sync);
+    if (s->cells_sync) cudaFree(s->cells_sync);
     if (s->direct) dst_plan_destroy(&s->dst);
     buf_free(s, s->flag);
     if (s->sync) cudaFree(s->sync);
@@ -337,6 +341,19 @@ int enqueue_poisson(cnv_state* s, const double* in, double scale, bool in_step) 
         static_assert(offsetof(Ctrl, status) == offsetof(Ctrl, iters) + 4 && offsetof(Ctrl, err) == offsetof(Ctrl, iters) + 8,
                       "Ctrl layout");
         CNV_CUDA(cudaMemsetAsync(reinterpret_cast<char*>(s->ctrl) + offsetof(Ctrl, iters), 0, 16, s->stream));
+        return CNV_OK;
+    }
+    if (s->cells.tc) {  // it writes the interior alone, as the direct solve does
+        CellsLaunch C{};
+        C.p = s->pp;
+        C.plan = s->cells;
+        for (int c = 0; c < 2; ++c) {
+            C.out[c] = s->sor[c];
+            C.rhs[c] = s->rhs[c];
+        }
+        C.ctrl = s->ctrl;
+        C.sync = s->cells_sync;
+        CNV_CUDA(launch_poisson_cells(C, s->stream));
         return CNV_OK;
     }
     if (s->tb) {
@@ -580,6 +597,14 @@ int cnv_create(const cnv_config* cfg, cnv_state** out) {
 #undef ALLOC
     // several sweeps per exchange: one block per SM, tiles at least as wide as the halo, the
     // psi tile (and the right-hand side when it also fits) in shared memory
+    if (!s->mixed && cfg->sor_blocking == 0 && cfg->solver_blocks <= 0 && cfg->test_stall_block == 0) {
+        s->cells = cells_plan(n, s->sms, prop.sharedMemPerBlockOptin, arith, cfg->poisson_type, fold);
+        cudaGetLastError();
+        if (s->cells.tc && cudaMalloc(&s->cells_sync, cells_sync_bytes(s->cells)) != cudaSuccess) {
+            free_state(s);
+            return fail(CNV_CUDA_ERROR, "cudaMalloc failed (solver mailboxes)");
+        }
+    }
     const int want_sweeps = cfg->sor_blocking == 0 ? auto_sor_sweeps(n) : cfg->sor_blocking;
     if (!s->mixed && cfg->poisson_type != CNV_POISSON_DIRECT && cfg->poisson_type != CNV_POISSON_JACOBI &&
         want_sweeps > 1) {
@@ -595,8 +620,8 @@ int cnv_create(const cnv_config* cfg, cnv_state** out) {
             s->tb = true;
             s->tb_g_smem = tb_smem_bytes(n, s->tb_gx, s->tb_gy, want_sweeps, true) + 2048 <= optin;
             const size_t snap = tb_snapshot_doubles(n, s->pitch);
-            if (buf_alloc(s, reinterpret_cast<void**>(&s->tb_snap), snap * sizeof(double), "s->tb_snap") != cudaSuccess ||
-                cudaMalloc(&s->tb_sync, tb_sync_bytes()) != cudaSuccess) {
+            if (s->cells.tc == 0 && (buf_alloc(s, reinterpret_cast<void**>(&s->tb_snap), snap * sizeof(double), "s->tb_snap") != cudaSuccess ||
+                cudaMalloc(&s->tb_sync, tb_sync_bytes()) != cudaSuccess)) {
                 free_state(s);
                 return fail(CNV_CUDA_ERROR, "cudaMalloc failed (tiled solver buffers)");
             }
@@ -918,6 +943,9 @@ int cnv_solver_info(cnv_state* s, char* buf, size_t len) {
                      s->tb_gx, s->tb_gy);
     else
         w = snprintf(buf, len, "sor-exchange grid=%d tiles=%dx%d", s->poisson_grid, s->poisson_gx, s->poisson_gy);
+    if (w >= 0 && (size_t)w < len && s->cells.tc)
+        w += snprintf(buf + w, len - w, "; run by sor-cells grid=%d tiles=%dx%d%s", s->cells.gx * s->cells.gy, s->cells.gx,
+                      s->cells.gy, s->cells.cluster ? " cluster" : "");
     if (w < 0 || (size_t)w >= len) return fail(CNV_BAD_ARG, "buffer of %zu bytes too small", len);
     return CNV_OK;
 }

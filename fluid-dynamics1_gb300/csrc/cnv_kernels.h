@@ -123,6 +123,27 @@ size_t tb_snapshot_doubles(int n, int pitch);
 size_t tb_smem_bytes(int n, int gx, int gy, int sweeps, bool g_smem);
 bool tb_tiles_ok(int n, int gx, int gy, int sweeps);
 
+// Red-black SOR / GS with a cell of each colour per thread (cnv_poisson_cells.cu): the same bits as launch_poisson, for small and
+// middle grids. out = the answer (split layout, zeroed edges), sync = cells_sync_bytes() (zeroed by the launch).
+struct CellsPlan {
+    int cluster;        // one cluster, mailboxes in shared memory
+    int gx, gy;
+    int norm_warps;
+    int tc, threads;    // compute threads and all threads of a block (tc 0: the kernel does not take the grid)
+    int side;           // cells of a mailbox side
+};
+struct CellsLaunch {
+    PoissonParams p;
+    CellsPlan plan;
+    double* out[2];
+    const double* rhs[2];
+    Ctrl* ctrl;
+    void* sync;
+};
+CellsPlan cells_plan(int n, int sms, size_t smem_max, Arith arith, int kind, bool fold);
+size_t cells_sync_bytes(const CellsPlan& plan);
+cudaError_t launch_poisson_cells(const CellsLaunch& L, cudaStream_t s);
+
 // Tile factorisation grid = gx * gy for an n x n grid (tiles near-square, at least 64 wide when
 // possible).
 void poisson_tiles(int n, int grid, int* gx, int* gy);
