@@ -123,14 +123,15 @@ size_t tb_snapshot_doubles(int n, int pitch);
 size_t tb_smem_bytes(int n, int gx, int gy, int sweeps, bool g_smem);
 bool tb_tiles_ok(int n, int gx, int gy, int sweeps);
 
-// Red-black SOR / GS with a cell of each colour per thread (cnv_poisson_cells.cu): the same bits as launch_poisson, for small and
-// middle grids. out = the answer (split layout, zeroed edges), sync = cells_sync_bytes() (zeroed by the launch).
+// Red-black SOR / GS with a cell of each colour per thread or tiles of many cells in shared memory (cnv_poisson_cells.cu): the
+// same bits as launch_poisson, up to 1100^2. out = the answer (split layout, zeroed edges), sync = cells_sync_bytes() (zeroed by the launch).
 struct CellsPlan {
     int cluster;        // one cluster, mailboxes in shared memory
     int gx, gy;
     int norm_warps;
     int tc, threads;    // compute threads and all threads of a block (tc 0: the kernel does not take the grid)
     int side;           // cells of a mailbox side
+    int rows, plane;    // tiles of many cells (rows 0: a cell of each colour per thread)
 };
 struct CellsLaunch {
     PoissonParams p;

@@ -304,8 +304,9 @@ int cnv_time_passes(cnv_state *s, int reps, double *pre_ms, double *post_ms);
 /* One line naming the Poisson solver this state runs and its geometry, e.g.
  * "sor-exchange grid=152 tiles=8x19" (FP64 SOR/GS exchanging every half-sweep),
  * "sor-tiled sweeps=4 grid=150 tiles=5x30" (several sweeps per exchange on shared-memory tiles), either
- * with "; run by sor-cells grid=16 tiles=4x4 cluster" where the default solve keeps a cell of each
- * colour per thread (the same bits) and the named kernel is what sor_blocking would pick, "mixed grid=152 tiles=8x19" or
+ * with "; run by sor-cells grid=16 tiles=4x4 cluster" where the default solve runs on registers or
+ * shared memory (the same bits) and the named kernel is the one that sor_blocking would pick,
+ * "mixed grid=152 tiles=8x19" or
  * "direct-sine-transform". Returns CNV_BAD_ARG if it does not fit in len bytes. */
 int cnv_solver_info(cnv_state *s, char *buf, size_t len);
 
