@@ -439,7 +439,7 @@ __device__ __forceinline__ unsigned long long fixed_of(float e0, int S) {
 // ------------------------------------------------------------------ the passes
 constexpr int kMaxMatrixRadix = 131;  // largest radix whose cosine and sine matrix is tabulated (36 KB)
 constexpr int kOneLaunchRows = 1300;  // largest m whose solve is one launch
-constexpr int kFp64Rows = 304;        // largest m solved in FP64 at once
+constexpr int kFp64Rows = 304;        // largest m solved in FP64 at once (fp64_radix_ok)
 constexpr int kThreads64 = 256;
 constexpr int kThreadsMax = 128;  // threads of a row's (column's) block
 
@@ -1173,6 +1173,20 @@ bool plan_fft(DstPlan* P, int a, int b, int sms, int smem_max, const Ctrl* ctrl,
     return true;
 }
 
+// Whether a transform of length len suits the FP64 form: its work grows with the largest prime factor p, which the FP32 form
+// does at FP32 rates. us per step, FP64 / FP32 (and the dense products of before): 135^2 (p = 67) 84.9 / 90.7 (113.7), 159^2 (79)
+// 95.5 / 94.6, 98^2 (97) 90.3 / 86.2, 202^2 (67) 109.7 / 103.6, 296^2 (59) 130.2 / 128.8, 200^2 (199) 299 / 149 (182).
+bool fp64_radix_ok(int len) {
+    int p = 1, rest = len;
+    for (int f = 2; f * f <= rest; ++f)
+        while (rest % f == 0) {
+            rest /= f;
+            p = std::max(p, f);
+        }
+    p = std::max(p, rest);
+    return p <= 61 || (p <= 79 && len <= 160);
+}
+
 }  // namespace
 
 int dst_plan_create(int n, int Lx, int Ly, Ctrl* ctrl, long long timeout_ns, DstPlan* P) {
@@ -1193,7 +1207,7 @@ int dst_plan_create(int n, int Lx, int Ly, Ctrl* ctrl, long long timeout_ns, Dst
     const int g = gcd(Lx, Ly);
     int status = CNV_OK;
     const DstPlan bare = *P;
-    if (m <= kFp64Rows) {
+    if (m <= kFp64Rows && fp64_radix_ok(m + 1)) {
         if (plan_fft<double>(P, Ly / g, Lx / g, sms, smem_max, ctrl, &status)) {
             if (status != CNV_OK) dst_plan_destroy(P);
             return status;

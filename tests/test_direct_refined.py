@@ -26,6 +26,7 @@ def solve(cnv, f, Lx=1, Ly=1):
 @pytest.mark.parametrize("n,Lx,Ly", [
     (5, 1, 1), (6, 1, 1), (12, 1, 1), (18, 1, 1), (33, 1, 1), (98, 1, 1), (129, 1, 1),  # N = 4, 5, 11, 17, 32, 97, 128
     (132, 1, 1), (138, 1, 1),    # N = 131, 137: the last tabulated radix, the first without a matrix
+    (80, 1, 1), (84, 1, 1), (159, 1, 1), (203, 1, 1), (200, 1, 40), (294, 1, 1),  # N = 79, 83, 158, 202, 199, 293: by radix
     (306, 1, 1), (307, 1, 1), (308, 1, 1),  # either side of the FP64 form's last size
     (514, 1, 1), (1026, 1, 1),   # N = 513 = 3^3 19, 1025 = 5^2 41
     (1302, 1, 1), (1303, 1, 1),  # the last size in one launch, the first launch per pass
