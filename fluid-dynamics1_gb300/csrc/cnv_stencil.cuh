@@ -62,6 +62,28 @@ __device__ __forceinline__ double along_i(const double (*band)[kTaps], int n, in
     return acc;
 }
 
+// The same sums where all seven taps lie inside the grid (class 3), x(o) the value at offset o, with fewer additions: 0.0 + p is p
+// (made +0 where p is -0), and the middle tap of a first derivative (ODD: its coefficient is 0) adds a zero to a sum that is
+// never -0, so it counts only where x(0) is not finite. The same bits for 22 instead of 28 additions in a cell's four
+// derivatives, and 20 instead of 28 in the velocity and continuity products.
+template <int MUL, bool ODD, class Load>
+__device__ __forceinline__ double inner_taps(const double (*band)[kTaps], Load x) {
+    const double* c = band[3];
+    double acc = band_mul<MUL>(c[0], x(-3));
+    if (((__double2hiint(acc) & 0x7fffffff) | __double2loint(acc)) == 0) acc = 0.0;
+    acc = dadd(acc, band_mul<MUL>(c[1], x(-2)));
+    acc = dadd(acc, band_mul<MUL>(c[2], x(-1)));
+    if (ODD) {
+        const double m = x(0);
+        if ((__double2hiint(m) & 0x7ff00000) == 0x7ff00000) acc = dadd(acc, dmul(c[3], m));
+    } else {
+        acc = dadd(acc, band_mul<MUL>(c[3], x(0)));
+    }
+    acc = dadd(acc, band_mul<MUL>(c[4], x(1)));
+    acc = dadd(acc, band_mul<MUL>(c[5], x(2)));
+    return dadd(acc, band_mul<MUL>(c[6], x(3)));
+}
+
 // Defect of the reference's discrete Poisson equation at one cell, in FP64 with an explicit
 // operation order (shared by the mixed-precision kernels so they agree bit for bit):
 //     R = g - (dy^2 (up + dn) + dx^2 (lt + rt) - den * p)

@@ -14,16 +14,15 @@
 // products are exact zeros). Velocity Dirichlet values (src/main.c:283-296) are applied on
 // read: u and v keep the values the velocity pass wrote, as in the reference between steps.
 //
-// k_pre. One block per 32 x 32 tile. The block stages w on its tile plus the radius-3 halo of
+// k_pre. One block per 32 x 8 tile. The block stages w on its tile plus the radius-3 halo of
 // the order-6 stencils in shared memory; cells on the grid's edge hold the new wall vorticity
 // there, which the block computes itself from u and v wherever its tile or halo touches an edge
-// (so no block reads another block's wall values). Each thread then takes four cells of one
-// column: the four derivatives from shared memory, u and v at the cell (coalesced global
+// (so no block reads another block's wall values). Each thread then takes one cell: the four derivatives from shared memory, u and v at the cell (coalesced global
 // loads), the Euler update, and the writes: w_out, the right-hand side in the solver's split
 // layout, and on edge cells the wall value into w_in (the reference's w after the wall loop,
 // which the adjoint form keeps).
 //
-// k_post. Persistent and cooperative: every block loops over 32 x 32 tiles. Phase 1 stages psi
+// k_post. Persistent and cooperative: every block loops over 32 x 8 tiles. Phase 1 stages psi
 // on the tile plus halo (from the solver's split layout) and writes u, v and the row-major psi
 // of the tile. A bounded grid barrier follows (continuity reads u and v of neighbouring tiles);
 // phase 2 stages u and v on the tile plus halo and reduces DX u + DY v to max and min. The
@@ -61,13 +60,14 @@ constexpr int kPostVel = kMulInt;    // k_post: DY psi, DX psi
 constexpr int kPostCont = kMulInt;   // k_post: DX u, DY v
 
 constexpr int kTX = 32;                 // tile columns (one warp across)
-// tile rows TY: 32 (each thread takes 4 cells of one column), or 8 on grids with fewer 32 x 32
-// tiles than twice the SM count (one cell per thread, four times the blocks: a 256^2 grid has
-// only 64 tiles of 32 x 32 for 152 SMs)
+// Tile rows, one cell per thread. Tiles of 32 rows (four cells per thread) stage fewer halo cells, but come in fewer blocks:
+// 1,024 of them at 1000^2 on 760 resident ones leave the last wave a third full. us, 32 rows / 8 rows: k_pre 500^2 63.5 / 45.9,
+// 1000^2 154 / 135, 2048^2 521 / 502; k_post 51.3 / 53.2, 130 / 124, 406 / 392.
+constexpr int kTY = 8;
 constexpr int kR = 3;                   // stencil radius (order 6; orders 2 and 4 use less)
 constexpr int kSW = kTX + 2 * kR;       // staged row width
-constexpr int kStepThreads = 256;       // 32 x 8: each thread takes 4 cells of one column
-constexpr int kThreadRows = kStepThreads / kTX;  // 8 rows of threads
+constexpr int kSH = kTY + 2 * kR;       // staged rows
+constexpr int kStepThreads = kTX * kTY;
 constexpr int kBandDoubles = (int)(sizeof(FdBands) / sizeof(double));
 
 __device__ __forceinline__ double make_rhs(double f_ref, const StepArgs& a) {
@@ -99,56 +99,66 @@ __device__ __forceinline__ double wall_value(const StepArgs& a, const FdBands& b
     return dsub(dvdx, dudy);
 }
 
+// All taps of a tile's columns, or of a row, inside the grid (the same for a whole warp).
+__device__ __forceinline__ bool inner_columns(int j0, int n) { return j0 >= kR && j0 + kTX <= n - kR; }
+__device__ __forceinline__ bool inner_row(int i, int n) { return i >= kR && i < n - kR; }
+
 __device__ __forceinline__ bool on_edge(int i, int j, int n) { return i == 0 || i == n - 1 || j == 0 || j == n - 1; }
 
 // ----------------------------------------------------------------------------------- k_pre
-template <int TY>
 __global__ void __launch_bounds__(kStepThreads) k_pre(StepArgs a) {
-    constexpr int kSH = TY + 2 * kR;  // staged rows
     if (a.ctrl->abort) return;
     __shared__ double sw[kSH * kSW];
     __shared__ FdBands sb;
     const int n = a.n;
-    const int j0 = blockIdx.x * kTX, i0 = blockIdx.y * TY;
+    const int j0 = blockIdx.x * kTX, i0 = blockIdx.y * kTY;
+    const int tx = threadIdx.x % kTX, ty = threadIdx.x / kTX, i = i0 + ty, j = j0 + tx;
+    const BoundaryValues bc = a.bc;
+    double ue = 0.0, ve = 0.0;  // asked for ahead of the staging
+    if (i < n && j < n) {
+        ue = vel_bc(a.u, n, i, j, bc.u1, bc.u2, bc.u3, bc.u4);
+        ve = vel_bc(a.v, n, i, j, bc.v1, bc.v2, bc.v3, bc.v4);
+    }
     stage_bands(sb, a.bands);
     __syncthreads();
     // w on the tile and halo; edge cells take the wall value
     const double* __restrict__ w = a.w_in;
     for (int x = threadIdx.x; x < kSH * kSW; x += kStepThreads) {
         const int r = x / kSW, c = x - r * kSW;
-        const int i = i0 - kR + r, j = j0 - kR + c;
+        const int y = i0 - kR + r, z = j0 - kR + c;
         double val = 0.0;
-        if (i >= 0 && i < n && j >= 0 && j < n) val = on_edge(i, j, n) ? wall_value(a, sb, i, j) : w[(size_t)i * n + j];
+        if (y >= 0 && y < n && z >= 0 && z < n) val = on_edge(y, z, n) ? wall_value(a, sb, y, z) : w[(size_t)y * n + z];
         sw[x] = val;
     }
     __syncthreads();
-    const int tx = threadIdx.x % kTX, ty = threadIdx.x / kTX;
-    const int j = j0 + tx;
-    if (j >= n) return;
+    if (i >= n || j >= n) return;
     auto W = [&](int r, int c) { return sw[(r - i0 + kR) * kSW + (c - j0 + kR)]; };
-    const BoundaryValues bc = a.bc;
-#pragma unroll 1
-    for (int k = 0; k < TY / kThreadRows; ++k) {
-        const int i = i0 + ty + k * kThreadRows;
-        if (i >= n) break;
-        const double wx = along_j<kPreD1>(sb.d1x, n, i, j, W);   // dwdx   = DX  w
-        const double wy = along_i<kPreD1>(sb.d1y, n, i, j, W);   // dwdy   = DY  w
-        const double wxx = along_j<kPreD2>(sb.d2x, n, i, j, W);  // d2wdx2 = DX2 w
-        const double wyy = along_i<kPreD2>(sb.d2y, n, i, j, W);  // d2wdy2 = DY2 w
-        const double ue = vel_bc(a.u, n, i, j, bc.u1, bc.u2, bc.u3, bc.u4);
-        const double ve = vel_bc(a.v, n, i, j, bc.v1, bc.v2, bc.v3, bc.v4);
-        const double w0 = W(i, j);
-        // (-u*dwdx - v*dwdy + (1./Re)*(d2wdx2 + d2wdy2))*dt + w   (src/fluiddyn.c:98)
-        const double conv = dsub(dmul(-ue, wx), dmul(ve, wy));
-        const double diff = dmul(a.inv_re, dadd(wxx, wyy));
-        const double wn = dadd(dmul(dadd(conv, diff), a.dt), w0);
-        const size_t at = (size_t)i * n + j;
-        a.w_out[at] = wn;
-        if (on_edge(i, j, n)) {
-            a.w_wall[at] = w0;  // the wall value, in place (src/main.c:311-320)
-        } else if (a.rhs[0]) {  // no rhs: the direct solve reads w_out itself
-            a.rhs[(i + j) & 1][(size_t)i * a.pitch + (j >> 1)] = make_rhs(-wn, a);  // f = -w (invsig)
-        }
+    double wx, wy, wxx, wyy;  // DX w, DY w, DX2 w, DY2 w
+    if (inner_columns(j0, n) && inner_row(i, n)) {
+        const double* at = &sw[(i - i0 + kR) * kSW + tx + kR];
+        auto J = [&](int o) { return at[o]; };
+        auto I = [&](int o) { return at[o * kSW]; };
+        wx = inner_taps<kPreD1, true>(sb.d1x, J);
+        wy = inner_taps<kPreD1, true>(sb.d1y, I);
+        wxx = inner_taps<kPreD2, false>(sb.d2x, J);
+        wyy = inner_taps<kPreD2, false>(sb.d2y, I);
+    } else {
+        wx = along_j<kPreD1>(sb.d1x, n, i, j, W);
+        wy = along_i<kPreD1>(sb.d1y, n, i, j, W);
+        wxx = along_j<kPreD2>(sb.d2x, n, i, j, W);
+        wyy = along_i<kPreD2>(sb.d2y, n, i, j, W);
+    }
+    const double w0 = W(i, j);
+    // (-u*dwdx - v*dwdy + (1./Re)*(d2wdx2 + d2wdy2))*dt + w   (src/fluiddyn.c:98)
+    const double conv = dsub(dmul(-ue, wx), dmul(ve, wy));
+    const double diff = dmul(a.inv_re, dadd(wxx, wyy));
+    const double wn = dadd(dmul(dadd(conv, diff), a.dt), w0);
+    const size_t at = (size_t)i * n + j;
+    a.w_out[at] = wn;
+    if (on_edge(i, j, n)) {
+        a.w_wall[at] = w0;  // the wall value, in place (src/main.c:311-320)
+    } else if (a.rhs[0]) {  // no rhs: the direct solve reads w_out itself
+        a.rhs[(i + j) & 1][(size_t)i * a.pitch + (j >> 1)] = make_rhs(-wn, a);  // f = -w (invsig)
     }
 }
 
@@ -159,11 +169,22 @@ struct Ext {
     int at;  // row-major index; -1 for the start value (which every tie keeps)
 };
 
+// Compared as integers, off the FP64 pipe (four comparisons a cell): sign and magnitude as one signed number, both zeros 0, and
+// no NaN taken.
+__device__ __forceinline__ long long order_of(double x) {
+    const long long b = __double_as_longlong(x);
+    return b >= 0 ? b : -(b & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ bool is_nan(double x) {
+    return (__double_as_longlong(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+}
 __device__ __forceinline__ void take_max(Ext& a, double v, int at) {
-    if (v > a.v || (v == a.v && at < a.at)) a = Ext{v, at};
+    const long long x = order_of(v), y = order_of(a.v);
+    if (!is_nan(v) && (x > y || (x == y && at < a.at))) a = Ext{v, at};
 }
 __device__ __forceinline__ void take_min(Ext& a, double v, int at) {
-    if (v < a.v || (v == a.v && at < a.at)) a = Ext{v, at};
+    const long long x = order_of(v), y = order_of(a.v);
+    if (!is_nan(v) && (x < y || (x == y && at < a.at))) a = Ext{v, at};
 }
 
 __device__ __forceinline__ void warp_ext(Ext& mx, Ext& mn) {
@@ -178,16 +199,14 @@ __device__ __forceinline__ void warp_ext(Ext& mx, Ext& mn) {
     }
 }
 
-template <int TY>
 __global__ void __launch_bounds__(kStepThreads) k_post(StepArgs a, int continuity) {
-    constexpr int kSH = TY + 2 * kR;  // staged rows
     if (a.ctrl->abort) return;  // stable for the whole launch: every block returns, or none
     __shared__ double sm[2 * kSH * kSW];  // phase 1: psi; phase 2: u and v
     __shared__ FdBands sb;
     __shared__ int s_ok;
     const int n = a.n;
     const int tiles_x = (n + kTX - 1) / kTX;
-    const int tiles = tiles_x * ((n + TY - 1) / TY);
+    const int tiles = tiles_x * ((n + kTY - 1) / kTY);
     const int tx = threadIdx.x % kTX, ty = threadIdx.x / kTX;
     stage_bands(sb, a.bands);
     __syncthreads();
@@ -197,27 +216,31 @@ __global__ void __launch_bounds__(kStepThreads) k_post(StepArgs a, int continuit
     const double* b = a.sor[1];
     const int pitch = a.pitch;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int j0 = (tile % tiles_x) * kTX, i0 = (tile / tiles_x) * TY;
+        const int j0 = (tile % tiles_x) * kTX, i0 = (tile / tiles_x) * kTY;
         for (int x = threadIdx.x; x < kSH * kSW; x += kStepThreads) {
             const int rr = x / kSW, c = x - rr * kSW;
             const int i = i0 - kR + rr, j = j0 - kR + c;
             sm[x] = (i >= 0 && i < n && j >= 0 && j < n) ? ((i + j) & 1 ? b : r)[(size_t)i * pitch + (j >> 1)] : 0.0;
         }
         __syncthreads();
+        const bool inner = inner_columns(j0, n);
         auto P = [&](int y, int c) { return sm[(y - i0 + kR) * kSW + (c - j0 + kR)]; };
         const int j = j0 + tx;
-        if (j < n) {
-#pragma unroll 1
-            for (int k = 0; k < TY / kThreadRows; ++k) {
-                const int i = i0 + ty + k * kThreadRows;
-                if (i >= n) break;
-                const double uu = along_i<kPostVel>(sb.d1y, n, i, j, P);   // DY psi
-                const double vv = -along_j<kPostVel>(sb.d1x, n, i, j, P);  // -(DX psi)
-                const size_t at = (size_t)i * n + j;
-                a.u[at] = uu;
-                a.v[at] = vv;
-                a.psi[at] = P(i, j);
+        const int i = i0 + ty;
+        if (j < n && i < n) {
+            double uu, vv;  // DY psi, -(DX psi)
+            if (inner && inner_row(i, n)) {
+                const double* at = &sm[(i - i0 + kR) * kSW + tx + kR];
+                uu = inner_taps<kPostVel, true>(sb.d1y, [&](int o) { return at[o * kSW]; });
+                vv = -inner_taps<kPostVel, true>(sb.d1x, [&](int o) { return at[o]; });
+            } else {
+                uu = along_i<kPostVel>(sb.d1y, n, i, j, P);
+                vv = -along_j<kPostVel>(sb.d1x, n, i, j, P);
             }
+            const size_t at = (size_t)i * n + j;
+            a.u[at] = uu;
+            a.v[at] = vv;
+            a.psi[at] = P(i, j);
         }
         __syncthreads();
     }
@@ -238,7 +261,7 @@ __global__ void __launch_bounds__(kStepThreads) k_post(StepArgs a, int continuit
     double* su = sm;
     double* sv = sm + kSH * kSW;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const int j0 = (tile % tiles_x) * kTX, i0 = (tile / tiles_x) * TY;
+        const int j0 = (tile % tiles_x) * kTX, i0 = (tile / tiles_x) * kTY;
         for (int x = threadIdx.x; x < kSH * kSW; x += kStepThreads) {
             const int rr = x / kSW, c = x - rr * kSW;
             const int i = i0 - kR + rr, j = j0 - kR + c;
@@ -247,20 +270,24 @@ __global__ void __launch_bounds__(kStepThreads) k_post(StepArgs a, int continuit
             sv[x] = in ? __ldcg(a.v + (size_t)i * n + j) : 0.0;
         }
         __syncthreads();
+        const bool inner = inner_columns(j0, n);
         auto U = [&](int y, int c) { return su[(y - i0 + kR) * kSW + (c - j0 + kR)]; };
         auto V = [&](int y, int c) { return sv[(y - i0 + kR) * kSW + (c - j0 + kR)]; };
         const int j = j0 + tx;
-        if (j < n) {
-#pragma unroll 1
-            for (int k = 0; k < TY / kThreadRows; ++k) {
-                const int i = i0 + ty + k * kThreadRows;
-                if (i >= n) break;
-                const double dudx = along_j<kPostCont>(sb.d1x, n, i, j, U);
-                const double dvdy = along_i<kPostCont>(sb.d1y, n, i, j, V);
-                const double c = dadd(dudx, dvdy);
-                take_max(mx, c, i * n + j);
-                take_min(mn, c, i * n + j);
+        const int i = i0 + ty;
+        if (j < n && i < n) {
+            double dudx, dvdy;
+            if (inner && inner_row(i, n)) {
+                const int at = (i - i0 + kR) * kSW + tx + kR;
+                dudx = inner_taps<kPostCont, true>(sb.d1x, [&](int o) { return su[at + o]; });
+                dvdy = inner_taps<kPostCont, true>(sb.d1y, [&](int o) { return sv[at + o * kSW]; });
+            } else {
+                dudx = along_j<kPostCont>(sb.d1x, n, i, j, U);
+                dvdy = along_i<kPostCont>(sb.d1y, n, i, j, V);
             }
+            const double c = dadd(dudx, dvdy);
+            take_max(mx, c, i * n + j);
+            take_min(mn, c, i * n + j);
         }
         __syncthreads();
     }
@@ -344,13 +371,31 @@ __global__ void k_nonfinite(const double* x, long long count, int* flag) {
 
 dim3 grid2d(int n, dim3 blk) { return dim3((n + blk.x - 1) / blk.x, (n + blk.y - 1) / blk.y); }
 
-int tile_count(int n, int ty) { return ((n + kTX - 1) / kTX) * ((n + ty - 1) / ty); }
+int tile_count(int n) { return ((n + kTX - 1) / kTX) * ((n + kTY - 1) / kTY); }
 
-template <int TY>
-cudaError_t launch_post_t(const StepArgs& a, bool continuity, cudaStream_t s) {
+}  // namespace
+
+cudaError_t launch_pre(const StepArgs& a, cudaStream_t s) {
+    k_pre<<<dim3((a.n + kTX - 1) / kTX, (a.n + kTY - 1) / kTY), kStepThreads, 0, s>>>(a);
+    return cudaGetLastError();
+}
+
+int post_grid(int n, int device) {
+    int sms = 0, per_sm = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_post, kStepThreads, 0) != cudaSuccess || per_sm < 1)
+        return 0;
+    // every block the same number of tiles: with more tiles than resident blocks, a grid of all
+    // resident blocks would leave some with one tile more than others in both phases
+    const int tiles = tile_count(n), resident = sms * per_sm;
+    const int per_block = (tiles + resident - 1) / resident;
+    return (tiles + per_block - 1) / per_block;
+}
+
+cudaError_t launch_post(const StepArgs& a, bool continuity, cudaStream_t s) {
     int c = continuity ? 1 : 0;
     if (!continuity) {  // no barrier: one block per tile
-        k_post<TY><<<tile_count(a.n, TY), kStepThreads, 0, s>>>(a, c);
+        k_post<<<tile_count(a.n), kStepThreads, 0, s>>>(a, c);
         return cudaGetLastError();
     }
     // the grid barrier needs every block resident: a cooperative launch of at most post_grid blocks
@@ -366,41 +411,7 @@ cudaError_t launch_post_t(const StepArgs& a, bool continuity, cudaStream_t s) {
     cfg.numAttrs = 1;
     StepArgs args = a;
     void* kargs[] = {&args, &c};
-    return cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(&k_post<TY>), kargs);
-}
-
-}  // namespace
-
-int step_tile_rows(int n, int device) {
-    int sms = 0;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || sms < 1) return 32;
-    return tile_count(n, 32) < 2 * sms ? 8 : 32;
-}
-
-cudaError_t launch_pre(const StepArgs& a, cudaStream_t s) {
-    if (a.tile_rows == 8)
-        k_pre<8><<<dim3((a.n + kTX - 1) / kTX, (a.n + 7) / 8), kStepThreads, 0, s>>>(a);
-    else
-        k_pre<32><<<dim3((a.n + kTX - 1) / kTX, (a.n + 31) / 32), kStepThreads, 0, s>>>(a);
-    return cudaGetLastError();
-}
-
-int post_grid(int n, int device, int tile_rows) {
-    int sms = 0, per_sm = 0;
-    const void* kern =
-        tile_rows == 8 ? reinterpret_cast<const void*>(&k_post<8>) : reinterpret_cast<const void*>(&k_post<32>);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kStepThreads, 0) != cudaSuccess || per_sm < 1)
-        return 0;
-    // every block the same number of tiles: with more tiles than resident blocks, a grid of all
-    // resident blocks would leave some with one tile more than others in both phases
-    const int tiles = tile_count(n, tile_rows == 8 ? 8 : 32), resident = sms * per_sm;
-    const int per_block = (tiles + resident - 1) / resident;
-    return (tiles + per_block - 1) / per_block;
-}
-
-cudaError_t launch_post(const StepArgs& a, bool continuity, cudaStream_t s) {
-    return a.tile_rows == 8 ? launch_post_t<8>(a, continuity, s) : launch_post_t<32>(a, continuity, s);
+    return cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(&k_post), kargs);
 }
 
 cudaError_t launch_to_split(const double* f, double* r, double* b, const StepArgs& a, cudaStream_t s) {
