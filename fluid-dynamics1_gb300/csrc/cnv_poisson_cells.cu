@@ -25,7 +25,7 @@
 // Stop test. Norm warps form the block's share of e_k from the ring (exact fixed-point sums, as in cnv_sor.cuh) while the
 // compute warps run on, and add it to a global ring whose words count the blocks in their upper bits: no fence, no counter, and
 // nothing is cleared (the verdict warps subtract what they read a turn before). A verdict warp in each block polls the words,
-// evaluates e_k and lets the compute warps run on: sweep k starts when e_{k - lag} is known, so every block stops before the
+// evaluates e_k and lets the compute warps run on: sweep k starts when e_{k - kLag} is known, so every block stops before the
 // same sweep, with the iterate of the one that converged still in the shared-memory ring. With a counter, fences and a cleared
 // slot per sweep the verdicts limited the pace (3,000 cycles a sweep at 64^2); with all blocks' atomics on one line they slowed the
 // mailboxes' traffic; gathered by one block and posted, the verdicts came too late (256^2: 2.87 ms a step, here 2.03).
@@ -44,12 +44,9 @@ namespace cnv {
 namespace {
 
 constexpr int kHist = 8;       // sweeps kept in shared memory
-// A sweep starts when the one `lag` before it is known not to have converged; what runs past the converged one is lost (512^2, a
-// solve of one sweep: 152 us with 6, 145 with 4), so the lag is what a verdict takes and no more: 6 sweeps of 1 us and more, or
-// 4 of 3.6 us and more with many cells (kLagMany; with 3 FMA 500^2 waited for it: 3.96 us a sweep against 3.58).
-constexpr int kLag = 6, kLagMany = 4;
+constexpr int kLag = 6;        // a sweep starts when the one kLag before it is known not to have converged
 static_assert(kHist > kLag, "the iterate that converged is still in the ring");
-constexpr int kNormRing = 32;  // sweeps' norms in flight: at least 3 lags (see check_norms)
+constexpr int kNormRing = 32;  // sweeps' norms in flight: at least 3 kLag (see check_norms)
 constexpr int kMinNormWarps = 2, kMaxNormWarps = 6;  // a whole sweep's share each, in turn
 
 // The norm's ring. A slot's words: the chunk sums of e_k for the k of that slot, all turns of the ring added up, over the blocks
@@ -344,9 +341,9 @@ __device__ void add_norms(const CellsDev& L, CellsShared& sh, const double* hist
 }
 
 // Verdict warp: the words of two sweeps at once (sixteen lanes a sweep, two words a lane), the complete ones judged in order. A
-// block adds its share of e_{j + kNormRing} after it knew e_{j + kNormRing - lag}, to which every block added after it knew
-// e_{j + kNormRing - 2 lag}, so after it read the slot of e_j. The side sums are cleared where they were used: block 0 clears the
-// slot of e_{j - lag} before it posts e_j (every block added to e_j after it knew e_{j - lag}).
+// block adds its share of e_{j + kNormRing} after it knew e_{j + kNormRing - kLag}, to which every block added after it knew
+// e_{j + kNormRing - 2 kLag}, so after it read the slot of e_j. The side sums are cleared where they were used: block 0 clears the
+// slot of e_{j - kLag} before it posts e_j (every block added to e_j after it knew e_{j - kLag}).
 template <int LAG>
 __device__ void check_norms(const CellsDev& L, CellsShared& sh) {
     static_assert(kNormRing >= 3 * LAG, "ring too short");
@@ -468,7 +465,6 @@ template <Arith A, int KIND, bool FOLD, bool INT, bool CLUSTER, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1) k_poisson_cells(CellsDev L) {
     extern __shared__ __align__(16) double hist[];  // [kHist][2][tc + 1]; then the mailboxes (CLUSTER)
     __shared__ CellsShared sh;
-    constexpr int LAG = MAXT > 640 ? kLagMany : kLag;
     Ctrl* ctl = L.ctrl;
     if (ctl->abort) return;  // stable for the whole launch: every block returns, or none
     const PoissonParams& p = L.p;
@@ -486,7 +482,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_poisson_cells(CellsDev L) {
     const int warp = tid >> 5, first_norm = tc >> 5;
     if (warp >= first_norm) {
         if (warp < first_norm + L.nw) add_norms(L, sh, hist, warp - first_norm);
-        else check_norms<LAG>(L, sh);
+        else check_norms<kLag>(L, sh);
     } else {
         int ci[2], cj[2];
         bool on[2];
@@ -521,17 +517,17 @@ __global__ void __launch_bounds__(MAXT, 1) k_poisson_cells(CellsDev L) {
                 bad = true;
                 break;
             }
-            if (k > LAG) {
+            if (k > kLag) {
                 unsigned long long gate;
                 for (;;) {  // by warp: the mailbox waits below need all lanes of one mind
                     gate = sh.gate;
-                    if (__all_sync(0xffffffffu, gate_checked(gate) >= k - LAG)) break;
+                    if (__all_sync(0xffffffffu, gate_checked(gate) >= k - kLag)) break;
                     if (__any_sync(0xffffffffu, sh.fail)) {
                         bad = true;
                         break;
                     }
                 }
-                if (!bad && gate_conv(gate) <= (unsigned)(k - LAG)) break;  // the same sweep in every thread of every block
+                if (!bad && gate_conv(gate) <= (unsigned)(k - kLag)) break;  // the same sweep in every thread of every block
             }
             double* now = hist + (k % kHist) * 2 * row;
             const double* before = hist + ((k - 1) % kHist) * 2 * row;
