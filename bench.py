@@ -185,11 +185,11 @@ class ClockSampler:
                 "samples": len(sm), "power_w_max": max(power) if power else None}
 
 
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one k_poisson launch on the headline
-# workload, from an ncu capture of the kernel as built at the commit named below. The solve runs
-# from L2, so this is the compulsory first touch of psi and f, not a per-sweep figure.
-POISSON_TRAFFIC = {"bytes_per_launch": 17982464.0,
-                   "source": "ncu capture of k_poisson, 1024^2 workload, one launch (step 0), build of commit f9d9c8a"}
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one k_poisson_rows launch at the headline
+# workload's size, from an ncu capture of the kernel as built at the commit named below. The solve runs from
+# shared memory, so this is the compulsory first touch of f (psi's write stays in L2), not a per-sweep figure.
+POISSON_TRAFFIC = {"bytes_per_launch": 9484288.0,
+                   "source": "ncu capture of k_poisson_rows, 1024^2, one launch of 600 sweeps, build of commit 0851c40"}
 
 L2_NOTE = "flushed before every timed step on the GPU (256 MB device write)"
 
@@ -535,10 +535,10 @@ def ours(args):
         # g, write R/den: 20 B) and update (read + write psi: 16 B)
         outer = sum(r["iters"] for r in recs)
         alg_bytes = interior * (12 * sweeps + 36 * outer)
-        kernel = "k_mixed (persistent FP32 red-black SOR in FP64 defect correction, one launch per step)"
+        kernel = "k_mixed_reg (persistent FP32 red-black SOR in FP64 defect correction, one launch per step)"
     else:
         alg_bytes = interior * BYTES_PER_CELL_SWEEP * sweeps
-        kernel = "k_poisson (persistent red-black SOR, one launch per step)"
+        kernel = "k_poisson_rows (persistent red-black SOR, one launch per step)"
     achieved = alg_bytes / (pms * 1e-3) / 1e9
     peak, peak_kind = measured_peaks()
     traffic = POISSON_TRAFFIC["bytes_per_launch"] if args.form == "fp64" else None
@@ -600,7 +600,7 @@ def ours(args):
                      "traffic_source": POISSON_TRAFFIC["source"] if traffic else None, "peak_source": peak_kind,
                      "kernel": kernel, "fp64_pipe": fp64},
         "e2e": e2e,
-        "gpu_launches": 3 * args.steps,  # k_pre, k_poisson, k_post per step
+        "gpu_launches": 3 * args.steps,  # k_pre, k_poisson_rows, k_post per step
         "step_passes": passes,
         "clocks": clk,
         "forms": forms,
