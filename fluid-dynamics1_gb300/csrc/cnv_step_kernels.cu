@@ -61,8 +61,9 @@ constexpr int kPostCont = kMulInt;   // k_post: DX u, DY v
 
 constexpr int kTX = 32;                 // tile columns (one warp across)
 // Tile rows, one cell per thread. Tiles of 32 rows (four cells per thread) stage fewer halo cells, but come in fewer blocks:
-// 1,024 of them at 1000^2 on 760 resident ones leave the last wave a third full. us, 32 rows / 8 rows: k_pre 500^2 63.5 / 45.9,
-// 1000^2 154 / 135, 2048^2 521 / 502; k_post 51.3 / 53.2, 130 / 124, 406 / 392.
+// 1,024 of them at 1000^2 on 760 resident ones leave the last wave a third full. us on a cavity at rest, 32 rows / 8 rows: k_pre 500^2
+// 63.5 / 45.9, 1000^2 154 / 135, 2048^2 521 / 502; k_post 51.3 / 53.2, 130 / 124, 406 / 392. On a developed field, with the shorter
+// sums (inner_taps) as well: k_pre 1024^2 111 -> 94, 2048^2 357 -> 339; k_post 134 -> 127, 430 -> 378.
 constexpr int kTY = 8;
 constexpr int kR = 3;                   // stencil radius (order 6; orders 2 and 4 use less)
 constexpr int kSW = kTX + 2 * kR;       // staged row width
