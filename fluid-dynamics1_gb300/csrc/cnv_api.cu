@@ -47,9 +47,8 @@ int fail(int status, const char* fmt, ...) {
                         __FILE__, __LINE__);                                                  \
     } while (0)
 
-// Sweeps per border exchange the FP64 SOR/GS solve uses by default for an n x n grid (1: the
-// kernel that exchanges every half-sweep; measured per sweep: 256^2 6.7 us tiled vs 8.6, 320^2
-// 12.3 vs 11.3, 512^2 11.4 vs 9.1, 768^2 31.5 vs 26.0).
+// Sweeps per border exchange of the FP64 SOR/GS solve on an n x n grid where cells_plan does not take it (forced block
+// counts, grids above 1100^2) and sor_blocking leaves the choice (1: the kernel that exchanges every half-sweep).
 // Sweeps per border exchange by grid size, from timings of both kernels on the cavity workload
 // (us per sweep, exchange kernel vs 2 / 4 sweeps per exchange): 256^2 7.38 vs 6.57 / 6.17,
 // 288^2 9.30 vs 8.90 / 8.85, 320^2 9.70 vs 9.42 / 10.12, 352^2 9.67 vs 10.11 / 10.99.
@@ -593,8 +592,7 @@ int cnv_create(const cnv_config* cfg, cnv_state** out) {
         }
     }
 #undef ALLOC
-    // several sweeps per exchange: one block per SM, tiles at least as wide as the halo, the
-    // psi tile (and the right-hand side when it also fits) in shared memory
+    // by default the kernels that keep the grid in registers or shared memory (a failed query there only means another kernel)
     if (!s->mixed && cfg->sor_blocking == 0 && cfg->solver_blocks <= 0 && cfg->test_stall_block == 0) {
         s->cells = cells_plan(n, s->sms, prop.sharedMemPerBlockOptin, arith, cfg->poisson_type, fold);
         cudaGetLastError();
@@ -603,6 +601,8 @@ int cnv_create(const cnv_config* cfg, cnv_state** out) {
             return fail(CNV_CUDA_ERROR, "cudaMalloc failed (solver mailboxes)");
         }
     }
+    // several sweeps per exchange: one block per SM, tiles at least as wide as the halo, the
+    // psi tile (and the right-hand side when it also fits) in shared memory
     const int want_sweeps = cfg->sor_blocking == 0 ? auto_sor_sweeps(n) : cfg->sor_blocking;
     if (!s->mixed && cfg->poisson_type != CNV_POISSON_DIRECT && cfg->poisson_type != CNV_POISSON_JACOBI &&
         want_sweeps > 1) {
