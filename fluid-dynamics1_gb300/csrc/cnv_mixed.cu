@@ -434,15 +434,19 @@ __device__ __forceinline__ pair_t fma2(pair_t a, pair_t b, pair_t c) {
     return r;
 }
 
-// Halo cells with their epoch: the eight bytes of a cell and its epoch arrive together, so a reader needs no flag, and the
-// writer no fence.
-__device__ __forceinline__ uint4 ld_relaxed4(const uint2* p) {
-    uint4 v;
-    asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+// Halo cells with their epoch: two cells per access, each a 64-bit word with the epoch above the value. A vector access is only
+// whole element by element, so the word, not the vector, is what keeps a value and its epoch together; a reader then needs no
+// flag, and the writer no fence.
+__device__ __forceinline__ ulonglong2 ld_cells(const uint2* p) {
+    ulonglong2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_relaxed4(uint2* p, uint4 v) {
-    asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+__device__ __forceinline__ void st_cells(uint2* p, unsigned long long a, unsigned long long b) {
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ unsigned long long tagged(unsigned value, unsigned epoch) {
+    return (unsigned long long)epoch << 32 | value;
 }
 
 extern __shared__ ulonglong2 mr_smem[];
@@ -695,7 +699,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_mixed_reg(MixedLaunch L) {
                 for (int h = 0; h < 2; ++h) {
                     const int i0 = row0 + h * PH;
                     if (own_col && i0 >= t.r0 && i0 + PH <= t.r1) continue;
-                    uint4 x[2][PH][2];
+                    ulonglong2 x[2][PH][2];
                     int polls = 0;
                     long long t0 = 0;
                     for (;;) {
@@ -705,7 +709,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_mixed_reg(MixedLaunch L) {
                             for (int k = 0; k < PH; ++k)
 #pragma unroll
                                 for (int v = 0; v < 2; ++v)
-                                    x[c][k][v] = ld_relaxed4(eg + ((size_t)(c ^ flip) * n + h * PH + k) * P + 2 * v);
+                                    x[c][k][v] = ld_cells(eg + ((size_t)(c ^ flip) * n + h * PH + k) * P + 2 * v);
                         bool there = true;
 #pragma unroll
                         for (int k = 0; k < PH; ++k) {
@@ -713,8 +717,9 @@ __global__ void __launch_bounds__(MAXT, 1) k_mixed_reg(MixedLaunch L) {
                             const bool want = i >= t.r0 - kHalo && i < t.r1 + kHalo && !(own_col && i >= t.r0 && i < t.r1);
                             unsigned d = 0;
 #pragma unroll
-                            for (int x4 = 0; x4 < 4; ++x4)
-                                d |= (x[x4 >> 1][k][x4 & 1].y ^ (ep - 1)) | (x[x4 >> 1][k][x4 & 1].w ^ (ep - 1));
+                            for (int v = 0; v < 4; ++v)
+                                d |= ((unsigned)(x[v >> 1][k][v & 1].x >> 32) ^ (ep - 1)) |
+                                     ((unsigned)(x[v >> 1][k][v & 1].y >> 32) ^ (ep - 1));
                             there = there && !(want && d);
                         }
                         if (there) break;
@@ -732,7 +737,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_mixed_reg(MixedLaunch L) {
 #pragma unroll
                         for (int k = 0; k < PH; ++k) {
                             if (own_col && i0 + k >= t.r0 && i0 + k < t.r1) continue;
-                            const unsigned v[PW] = {x[c][k][0].x, x[c][k][0].z, x[c][k][1].x, x[c][k][1].z};
+                            const unsigned v[PW] = {(unsigned)x[c][k][0].x, (unsigned)x[c][k][0].y, (unsigned)x[c][k][1].x, (unsigned)x[c][k][1].y};
 #pragma unroll
                             for (int u = 0; u < PW; ++u) {
                                 pair_t& E1 = E[c][k][u];
@@ -771,7 +776,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_mixed_reg(MixedLaunch L) {
 #pragma unroll
                                 for (int v = 0; RREG && v < S::kV; ++v) {
                                     const pair_t a = E[c][k][2 * v], b = E[c][k][2 * v + 1];
-                                    st_relaxed4(d + 2 * v, make_uint4((unsigned)(h ? a >> 32 : a), ep, (unsigned)(h ? b >> 32 : b), ep));
+                                    st_cells(d + 2 * v, tagged((unsigned)(h ? a >> 32 : a), ep), tagged((unsigned)(h ? b >> 32 : b), ep));
                                 }
                             }
                         }
