@@ -469,7 +469,7 @@ int cnv_adjoint_create(const cnv_config* cfg, int checkpoint_every, cnv_adjoint*
         return afail(CNV_BAD_ARG, "finite-difference bands");
     }
     if (cudaMemcpy(a->bands, &hb, sizeof hb, cudaMemcpyHostToDevice) != cudaSuccess) return bad("band upload");
-    if (dst_plan_create(n, cfg->Lx, cfg->Ly, a->ctrl, 2000000000LL, &a->dst) != CNV_OK) return bad("sine-transform plan");
+    if (dst_plan_create(n, cfg->Lx, cfg->Ly, a->ctrl, 2000000000LL, -1, &a->dst) != CNV_OK) return bad("sine-transform plan");
     // initial velocities of src/main.c:213-221: ui, vi on the interior, zero on the edges
     std::vector<double> hu(nn, 0.0), hv(nn, 0.0);
     for (int i = 1; i < n - 1; ++i)

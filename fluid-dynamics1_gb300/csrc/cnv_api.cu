@@ -330,15 +330,12 @@ MixedLaunch mixed_launch(cnv_state* s) {
 
 // Enqueue the Poisson solve on the split-layout rhs, or on g for the mixed form (psi starts
 // from zero). The direct solve reads the row-major field `in` scaled by `scale` instead
-// (w with c4 in a step, f with -c4 for a standalone solve) and reports 0 iterations.
+// (w with c4 in a step, f with -c4 for a standalone solve) and reports 0 iterations: the zeros of reset_ctrl, to which
+// it only ever adds the status of a wait that ran out.
 int enqueue_poisson(cnv_state* s, const double* in, double scale, bool in_step) {
     const size_t split_bytes = (size_t)s->n * s->pitch * 8;
     if (s->direct) {  // it writes the interior alone: the edges keep upload_initial's zeros
         CNV_CUDA(dst_solve_split(s->dst, in, scale, s->sor[0], s->sor[1], s->pitch, s->stream));
-        // iters, status (int) and err (double) of the control block: 0, CNV_OK, 0.0
-        static_assert(offsetof(Ctrl, status) == offsetof(Ctrl, iters) + 4 && offsetof(Ctrl, err) == offsetof(Ctrl, iters) + 8,
-                      "Ctrl layout");
-        CNV_CUDA(cudaMemsetAsync(reinterpret_cast<char*>(s->ctrl) + offsetof(Ctrl, iters), 0, 16, s->stream));
         return CNV_OK;
     }
     if (s->cells.tc) {  // it writes the interior alone, as the direct solve does
@@ -634,7 +631,8 @@ int cnv_create(const cnv_config* cfg, cnv_state** out) {
     if (cfg->poisson_type == CNV_POISSON_DIRECT) {
         s->direct = true;
         if (dst_plan_create(n, cfg->Lx, cfg->Ly, s->ctrl,
-                            (cfg->solver_timeout_ms > 0 ? cfg->solver_timeout_ms : 2000) * 1000000LL, &s->dst) != CNV_OK) {
+                            (cfg->solver_timeout_ms > 0 ? cfg->solver_timeout_ms : 2000) * 1000000LL,
+                            cfg->test_stall_block - 1, &s->dst) != CNV_OK) {
             free_state(s);
             return fail(CNV_CUDA_ERROR, "sine-transform plan for n = %d", n);
         }
@@ -906,7 +904,10 @@ int cnv_poisson_device(cnv_state* s, const double* f, double* psi_out, int* iter
     s->last_sweeps = h.sweeps;
     if (iters) *iters = h.iters;
     if (err) *err = h.err;
-    if (h.status != CNV_OK) return fail(h.status, "Poisson solve status %d", h.status);
+    if (h.abort || h.status != CNV_OK) {
+        const int status = h.status != CNV_OK ? h.status : CNV_CUDA_ERROR;
+        return fail(status, "Poisson solve status %d", status);
+    }
     return check_guards(s);
 }
 

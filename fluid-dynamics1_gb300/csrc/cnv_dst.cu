@@ -702,6 +702,7 @@ struct GridBarrier {
     int* ctl;
     Ctrl* ctrl;
     long long timeout_ns;
+    int stall_block;
     unsigned arrivals;
     __device__ __forceinline__ bool wait() {
         __shared__ int s_ok;
@@ -710,7 +711,7 @@ struct GridBarrier {
         arrivals += gridDim.x;
         if (threadIdx.x == 0) {
             __threadfence();
-            atomicAdd(count, 1u);
+            if ((int)blockIdx.x != stall_block) atomicAdd(count, 1u);
             s_ok = wait_geq(count, arrivals, ctrl, timeout_ns) ? 1 : 0;
         }
         __syncthreads();
@@ -725,12 +726,12 @@ struct GridBarrier {
 // All passes of a solve in one cooperative launch, block b taking row b + 1 and column b + 1, with a grid barrier between passes.
 template <int FORM>
 __global__ void __launch_bounds__(kThreadsMax, blocks_per_sm(FORM))
-    k_dst_all(FftArgs F, int solves, const double* in, KScale ks, DstDest dst, Ctrl* ctrl, long long timeout_ns) {
+    k_dst_all(FftArgs F, int solves, const double* in, KScale ks, DstDest dst, Ctrl* ctrl, long long timeout_ns, int stall_block) {
     extern __shared__ float2 fsm[];
     __shared__ int s_red[8];
     if (ctrl->abort) return;
     const Tables<float> tab = begin_pass<float, FORM == kSmall>(F, reinterpret_cast<float4*>(fsm + F.fields));
-    GridBarrier bar{F.ctl, ctrl, timeout_ns, 0};
+    GridBarrier bar{F.ctl, ctrl, timeout_ns, stall_block, 0};
     const int i = 1 + blockIdx.x;
     int E = 0, S = 0;
     for (int k = 0; k < solves; ++k) {
@@ -751,14 +752,14 @@ __global__ void __launch_bounds__(kThreadsMax, blocks_per_sm(FORM))
 // passes in launches of their own took 58); at 256^2 a step takes 15 % less than with the FP32 form. It lasts while an SM has
 // no more than two rows (kFp64Rows): the FP64 work of a third costs more than the FP32 form's further passes.
 __global__ void __launch_bounds__(kThreads64)
-    k_dst_fp64(FftArgs F, const double* in, double scale, DstDest dst, Ctrl* ctrl, long long timeout_ns) {
+    k_dst_fp64(FftArgs F, const double* in, double scale, DstDest dst, Ctrl* ctrl, long long timeout_ns, int stall_block) {
     extern __shared__ double2 dsm[];
     if (ctrl->abort) return;
     const int N = F.len, m = F.m, ld = F.ld, half = N / 2 + 1, nl = (m >> 1) + 1, i = 1 + blockIdx.x;
     double2* X = dsm;
     double2* T = dsm + N;
     const Tables<double> tab = begin_pass<double, true>(F, reinterpret_cast<float4*>(dsm + F.fields));
-    GridBarrier bar{F.ctl, ctrl, timeout_ns, 0};
+    GridBarrier bar{F.ctl, ctrl, timeout_ns, stall_block, 0};
     // along j
     const double* row = in + (size_t)i * F.n;
     for (int j = threadIdx.x; j < half; j += blockDim.x)
@@ -933,10 +934,10 @@ cudaError_t solve(const DstPlan& P, const double* in, double scale, const DstDes
         const KScale ks = multiplier(scale, P.kappa);
         const int blocks_b = ceil_div(m + 1, F.cols_b);  // modes 0 .. m; mode 0 is padding
         if (P.fp64)
-            return launch_pass(k_dst_fp64, m, kThreads64, P.smem_a, true, s, F, in, scale, d, P.ctrl, P.timeout_ns);
+            return launch_pass(k_dst_fp64, m, kThreads64, P.smem_a, true, s, F, in, scale, d, P.ctrl, P.timeout_ns, P.stall_block);
         if (P.one_launch) {
             const auto k1 = P.form == kSmall ? k_dst_all<kSmall> : P.form == kMid ? k_dst_all<kMid> : k_dst_all<kWide>;
-            return launch_pass(k1, m, P.threads_a, P.smem_a, true, s, F, P.solves, in, ks, d, P.ctrl, P.timeout_ns);
+            return launch_pass(k1, m, P.threads_a, P.smem_a, true, s, F, P.solves, in, ks, d, P.ctrl, P.timeout_ns, P.stall_block);
         }
         for (int k = 0; k < P.solves; ++k) {
             const auto ka = P.form == kSmall ? k_dst_a<kSmall> : P.form == kMid ? k_dst_a<kMid> : k_dst_a<kWide>;
@@ -1189,10 +1190,11 @@ bool fp64_radix_ok(int len) {
 
 }  // namespace
 
-int dst_plan_create(int n, int Lx, int Ly, Ctrl* ctrl, long long timeout_ns, DstPlan* P) {
+int dst_plan_create(int n, int Lx, int Ly, Ctrl* ctrl, long long timeout_ns, int stall_block, DstPlan* P) {
     *P = DstPlan{};
     P->ctrl = ctrl;
     P->timeout_ns = timeout_ns;
+    P->stall_block = stall_block;
     if (n < 3 || Lx < 1 || Ly < 1) return CNV_BAD_ARG;
     const int m = n - 2;
     const double dx = (double)Lx / n, dy = (double)Ly / n;

@@ -54,6 +54,7 @@ struct DstPlan {
     bool fp64 = false;         // in FP64 at once (small grids)
     Ctrl* ctrl = nullptr;
     long long timeout_ns = 0;
+    int stall_block = -1;      // testing only: a block of the one-launch forms that never arrives at their barriers
     int solves = 3;            // FP32 solves, each of the residual the ones before left
     double kappa = 1;          // the equation's operator over the integer stencil
     int rows = 4;              // rows per block of the dense product kernel
@@ -66,8 +67,8 @@ struct DstPlan {
 };
 
 // Lx and Ly are the cavity's extents (dx = Lx / n, dy = Ly / n). ctrl (may be null) takes the status and the abort flag
-// of a solve whose blocks wait for one another (bounded by timeout_ns).
-int dst_plan_create(int n, int Lx, int Ly, Ctrl* ctrl, long long timeout_ns, DstPlan* plan);
+// of a solve whose blocks wait for one another (bounded by timeout_ns). stall_block: see DstPlan (-1: none).
+int dst_plan_create(int n, int Lx, int Ly, Ctrl* ctrl, long long timeout_ns, int stall_block, DstPlan* plan);
 // Re-arm the barrier after a solve that timed out: once before the solves of a call.
 cudaError_t dst_reset(const DstPlan& plan, cudaStream_t s);
 void dst_plan_destroy(DstPlan* plan);

@@ -138,7 +138,7 @@ struct PoissonParams {
     MulConst kb4, komb;  // b4 and omb for the folded form's integer multiply
     int fold;           // 1: exact form with power-of-two scalings folded (dx = dy, dx^2 and den powers of 2)
     long long timeout_ns;  // bound on every wait for another block
-    int stall_block;       // testing only: block of the exchange kernel that never raises its flags (-1: none)
+    int stall_block;       // testing only: a block that never raises its flags (-1: none)
 };
 
 // Set the text cnv_last_error() returns on this thread.

@@ -104,7 +104,8 @@ typedef struct cnv_config {
                                 step's psi instead of zero (same stop rule: FP64 relative residual) */
     int solver_timeout_ms;   /* bound on every on-device wait for another block; <= 0: 2000 */
     int test_stall_block;    /* testing only: 1 + the index of a block of the FP64 SOR/GS exchange
-                                kernel that never raises its progress flags, so that its neighbours'
+                                kernel that never raises its progress flags, or of the direct solve
+                                in one launch that never arrives at its barriers, so that the others'
                                 bounded waits run out (the solve returns CNV_TIMEOUT); 0: off */
     int test_guard_cells;    /* testing only: 1 puts 4 KB of 0xFF bytes (NaN in every lane width)
                                 before and after every field and work buffer and checks them after
