@@ -239,6 +239,13 @@ int end_run(cnv_adjoint* a) {
     return h.abort ? afail(h.status != CNV_OK ? h.status : CNV_CUDA_ERROR, "grid barrier wait timed out") : CNV_OK;
 }
 
+// The same after a forward run: one that gave up leaves no states to differentiate.
+int end_forward(cnv_adjoint* a) {
+    const int rc = end_run(a);
+    if (rc != CNV_OK) a->steps = -1;
+    return rc;
+}
+
 size_t nn_of(const cnv_adjoint* a) { return (size_t)a->n * a->n; }
 
 double* slot_w(double* base, size_t nn, size_t k) { return base + 3 * nn * k; }
@@ -255,6 +262,9 @@ int ensure_slots(GuardSet& guards, double** buf, size_t* have, size_t want, size
     return CNV_OK;
 }
 
+// Bound on a wait for another block.
+long long timeout_ns_of(const cnv_config& c) { return (c.solver_timeout_ms > 0 ? c.solver_timeout_ms : 2000) * 1000000LL; }
+
 StepArgs base_args(const cnv_adjoint* a) {
     StepArgs s{};
     s.n = a->n;
@@ -269,7 +279,7 @@ StepArgs base_args(const cnv_adjoint* a) {
     s.sor[0] = a->sor[0];
     s.sor[1] = a->sor[1];
     s.ctrl = a->ctrl;
-    s.timeout_ns = 2000000000LL;
+    s.timeout_ns = timeout_ns_of(c);
     return s;
 }
 
@@ -469,7 +479,8 @@ int cnv_adjoint_create(const cnv_config* cfg, int checkpoint_every, cnv_adjoint*
         return afail(CNV_BAD_ARG, "finite-difference bands");
     }
     if (cudaMemcpy(a->bands, &hb, sizeof hb, cudaMemcpyHostToDevice) != cudaSuccess) return bad("band upload");
-    if (dst_plan_create(n, cfg->Lx, cfg->Ly, a->ctrl, 2000000000LL, -1, &a->dst) != CNV_OK) return bad("sine-transform plan");
+    if (dst_plan_create(n, cfg->Lx, cfg->Ly, a->ctrl, timeout_ns_of(*cfg), cfg->test_stall_block - 1, &a->dst) != CNV_OK)
+        return bad("sine-transform plan");
     // initial velocities of src/main.c:213-221: ui, vi on the interior, zero on the edges
     std::vector<double> hu(nn, 0.0), hv(nn, 0.0);
     for (int i = 1; i < n - 1; ++i)
@@ -494,7 +505,7 @@ int cnv_adjoint_forward_device(cnv_adjoint* a, const double* w0, double lid, int
     if (rc != CNV_OK) return rc;
     if (w_final)
         ACUDA(cudaMemcpyAsync(w_final, a->w[a->cur], nn_of(a) * 8, cudaMemcpyDeviceToDevice, a->stream));
-    if ((rc = end_run(a)) != CNV_OK) return rc;
+    if ((rc = end_forward(a)) != CNV_OK) return rc;
     float ms = 0;
     cudaEventElapsedTime(&ms, a->ev[0], a->ev[1]);
     a->fwd_ms = ms;
@@ -518,7 +529,7 @@ int cnv_adjoint_forward(cnv_adjoint* a, const double* w0, double lid, int nsteps
     if (rc != CNV_OK) return rc;
     std::vector<double> h(nn);
     ACUDA(cudaMemcpyAsync(h.data(), a->w[a->cur], nn * 8, cudaMemcpyDeviceToHost, a->stream));
-    if ((rc = end_run(a)) != CNV_OK) return rc;
+    if ((rc = end_forward(a)) != CNV_OK) return rc;
     float ms = 0;
     cudaEventElapsedTime(&ms, a->ev[0], a->ev[1]);
     a->fwd_ms = ms;

@@ -35,3 +35,20 @@ def test_a_block_that_never_publishes_is_reported(cnv, n, kw):
     with cnv.Cavity(make_cfg(cnv, n, **limits)) as cav:
         rc, psi, it2, err2 = cav.poisson(f)
     assert (rc, it2, err2) == (0, it, err) and np.array_equal(psi, want)
+
+
+@pytest.mark.parametrize("n", [64, 400])
+def test_a_forward_run_that_gave_up_cannot_be_differentiated(cnv, n):
+    h = 1.0 / n
+    cfg = cnv.default_config(nx=n, ny=n, Re=400.0, dt=0.2 * min(h * h * 100.0, h), solver_timeout_ms=50, test_stall_block=1 + 3)
+    w0 = cnv.noise_field(n, seed=5, sigma=1.0, passes=4)
+    with cnv.Adjoint(cfg, 2) as adj:
+        t0 = time.perf_counter()
+        for _ in range(2):
+            with pytest.raises(cnv.CnvError) as e:
+                adj.forward(w0, 1.0, 3)
+            assert e.value.status == cnv.CNV_TIMEOUT
+            with pytest.raises(cnv.CnvError) as e:
+                adj.backward(w0)
+            assert e.value.status == cnv.CNV_BAD_ARG
+        assert time.perf_counter() - t0 < 1.0  # solver_timeout_ms, not the default of two seconds
