@@ -20,14 +20,15 @@
 //     with integer coefficients.
 //   - psi is held as 64-bit fixed point: psi = I 2^(E-1023-S) scale / kappa, with E the largest biased exponent
 //     of `in` and S such that the largest |I| is about 2^58. In these units the right-hand side is in * 2^(S-E+1023),
-//     an exponent shift of the double, and the residual in * 2^.. - (a^2 Di + b^2 Dj) I is a sum of 64-bit integers. It is
-//     taken modulo 2^64, which is exact because the residual itself is small; only the right-hand side is rounded
-//     (to one unit, 2^-58 of the largest |psi|).
+//     an exponent shift of the double, and the residual in * 2^.. - (a^2 Di + b^2 Dj) I is a sum of 64-bit integers and
+//     the right-hand side's fraction. The integers are taken modulo 2^64, which is exact because the residual itself is small;
+//     the fraction is added to them as a float. (A unit is 2^-58 of the largest |psi|, and psi is up to 0.07 n^2 times the
+//     right-hand side: without the fraction, cells of one value, all rounded alike, put psi off by 6e-14 at 1000^2, 2e-13 at 2048^2.)
 //   - The first FP32 solve starts from `in`, each later one from the residual, and adds to I. A solve leaves about
-//     3e-7 of the answer, the next 1e-11 .. 1e-10, the third less than the rounding of psi to FP64 (modelled in numpy
-//     with this arithmetic against an extended-precision solve, n = 5 .. 4097: 5e-18 .. 8e-16; an FP64 sine-transform
-//     solve has 3e-16 .. 8e-16). Where the estimate of the third is above 1e-16 (long transforms, large radices, stretched
-//     cells) a fourth is made.
+//     3e-7 of the answer, the next 1e-11 .. 1e-10, the third less than the rounding of psi to FP64 for most right-hand sides
+//     (against extended-precision solves, n = 200 .. 4097: noise, a point and smooth ones 6e-17 .. 1e-15, a constant and
+//     a disc of one value up to 4e-15, at 4097^2; FP64 sine transforms: 5e-16 .. 1e-13). Where the estimate of the third is
+//     above 1e-16 (long transforms, large radices, stretched cells) a fourth is made.
 //   - I times scale / kappa is rounded once to FP64, in integer arithmetic.
 // The residual is part of the next solve's first pass and the addition of the last one, so a solve is three
 // launches: A rows (residual, transform along j), B columns (transform along i, divide by the eigenvalues, transform
@@ -380,17 +381,20 @@ __device__ __forceinline__ float scaled_float(double x, int E) {
     return __uint_as_float((((unsigned)e << 23) | m) + ((lo >> 28) & 1u) | (hi & 0x80000000u));
 }
 
-// x * 2^(1023 - E + S), rounded to an integer (half up in magnitude), modulo 2^64. Without branches:
-// neighbouring cells take either side.
-__device__ __forceinline__ unsigned long long scaled_int(double x, int E, int S) {
+// x * 2^(1023 - E + S), rounded to an integer (half up in magnitude), modulo 2^64; `rest` takes what the rounding left out, between
+// -1/2 and 1/2. Without branches: neighbouring cells take either side.
+__device__ __forceinline__ unsigned long long scaled_int(double x, int E, int S, float& rest) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(x);
     const int f = (int)((b >> 52) & 0x7ff);
-    const unsigned long long m = (b & ((1ull << 52) - 1)) | (f ? 1ull << 52 : 0ull);
+    unsigned long long m = (b & ((1ull << 52) - 1)) | (f ? 1ull << 52 : 0ull);
     const int sh = max(f, 1) - E - 52 + S;
+    m >>= min(max(-53 - sh, 0), 63);         // below half a unit: all of it is rest
     const int r = min(max(10 - sh, 1), 63);  // right shift of m << 10
-    const unsigned long long right = ((m << 10) + (1ull << (r - 1))) >> r;
+    const unsigned long long q = (m << 10) + (1ull << (r - 1));
     const unsigned long long left = sh < 64 ? m << max(min(sh, 63), 0) : 0ull;
-    const unsigned long long v = sh < 10 ? right : left;
+    const unsigned long long v = sh < 10 ? q >> r : left;
+    const float below = fmaf((float)(unsigned)((q << (64 - r)) >> 32), 0x1p-32f, -0.5f);  // (0 for sh >= 0)
+    rest = (long long)b < 0 ? -below : below;
     return (long long)b < 0 ? 0ull - v : v;
 }
 
@@ -546,8 +550,9 @@ __device__ __forceinline__ void pass_a(const FftArgs& F, const Tables<float>& ta
                         v = field<ONE>(p + ld) + field<ONE>(p - ld);
                         h = field<ONE>(p + 1) + field<ONE>(p - 1);
                     }
-                    const unsigned long long g = scaled_int(row[jj], E, S);
-                    y[q] = float_of(unit ? g - 4 * c + v + h : g - ab * c + a2 * v + b2 * h);
+                    float rest;
+                    const unsigned long long g = scaled_int(row[jj], E, S, rest);
+                    y[q] = float_of(unit ? g - 4 * c + v + h : g - ab * c + a2 * v + b2 * h) + rest;
                 }
             }
             put_z<1, float>(F, tab, X, j, 0, y[0], y[1]);
