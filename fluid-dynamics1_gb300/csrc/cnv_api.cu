@@ -315,6 +315,7 @@ MixedLaunch mixed_launch(cnv_state* s) {
     L.ntx = s->mixed_ntx;
     L.nty = s->mixed_nty;
     L.timeout_ns = s->pp.timeout_ns;
+    L.stall_block = s->pp.stall_block;
     const size_t split = (size_t)s->n * s->pitch;
     for (int c = 0; c < 2; ++c) {
         L.g[c] = s->rhs[c];
@@ -590,7 +591,7 @@ int cnv_create(const cnv_config* cfg, cnv_state** out) {
     }
 #undef ALLOC
     // by default the kernels that keep the grid in registers or shared memory (a failed query there only means another kernel)
-    if (!s->mixed && cfg->sor_blocking == 0 && cfg->solver_blocks <= 0 && cfg->test_stall_block == 0) {
+    if (!s->mixed && cfg->sor_blocking == 0 && cfg->solver_blocks <= 0) {
         s->cells = cells_plan(n, s->sms, prop.sharedMemPerBlockOptin, arith, cfg->poisson_type, fold);
         cudaGetLastError();
         if (s->cells.tc && cudaMalloc(&s->cells_sync, cells_sync_bytes(s->cells)) != cudaSuccess) {

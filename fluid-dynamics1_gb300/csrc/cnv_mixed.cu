@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_mixed(MixedLaunch L) {
                     L.eg[par][c][(size_t)i * P + (j >> 1)] = S.at(c, i, j >> 1);
                 }
                 __syncthreads();
-                if (threadIdx.x == 0) st_release(&sy->flag[blockIdx.x], ep);
+                if (threadIdx.x == 0 && (int)blockIdx.x != L.stall_block) st_release(&sy->flag[blockIdx.x], ep);
             }
         }
         if (!ok) { status = CNV_TIMEOUT; break; }
@@ -757,7 +757,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_mixed_reg(MixedLaunch L) {
             sweeps += kSweepsPerExchange;
             if (e + 1 < L.epochs) {
                 // own cells near the tile's border -> global copy of this epoch, each with the epoch
-                if (p.on && own_col) {
+                if (p.on && own_col && (int)blockIdx.x != L.stall_block) {
                     uint2* eg = L.eg2 + (size_t)(ep & 1) * 2 * n * P + mt;
 #pragma unroll
                     for (int h = 0; h < 2; ++h)
@@ -783,7 +783,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_mixed_reg(MixedLaunch L) {
                 }
                 if (!RREG) {
                     __syncthreads();
-                    if (threadIdx.x == 0) st_release(&sy->flag[blockIdx.x], ep);
+                    if (threadIdx.x == 0 && (int)blockIdx.x != L.stall_block) st_release(&sy->flag[blockIdx.x], ep);
                 }
             }
         }

@@ -478,6 +478,10 @@ __global__ void __launch_bounds__(MAXT, 1) k_poisson_cells(CellsDev L) {
     cells_clear(sh);
     __syncthreads();
     if (CLUSTER) cooperative_groups::this_cluster().sync();
+    if (me == p.stall_block) {  // tests only: a block that does nothing but stay until the others have given up
+        if (CLUSTER) cooperative_groups::this_cluster().sync();
+        return;
+    }
 
     const int warp = tid >> 5, first_norm = tc >> 5;
     if (warp >= first_norm) {
@@ -663,6 +667,7 @@ __global__ void __launch_bounds__(MAXT + 64, 1) k_poisson_rows(CellsDev L) {
     cells_clear(sh);
     if (tid < 4) rs.side[tid] = 0;
     __syncthreads();
+    if (me == p.stall_block) return;  // tests only: a block that does nothing
 
     if (warp == tc / 32) {
         add_row_norms(L, sh, rs);

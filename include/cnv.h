@@ -103,10 +103,11 @@ typedef struct cnv_config {
     int mixed_warm_start;    /* CNV_PREC_MIXED (and batches): start each step's solve from the previous
                                 step's psi instead of zero (same stop rule: FP64 relative residual) */
     int solver_timeout_ms;   /* bound on every on-device wait for another block; <= 0: 2000 */
-    int test_stall_block;    /* testing only: 1 + the index of a block of the FP64 SOR/GS exchange
-                                kernel that never raises its progress flags, or of the direct solve
-                                in one launch that never arrives at its barriers, so that the others'
-                                bounded waits run out (the solve returns CNV_TIMEOUT); 0: off */
+    int test_stall_block;    /* testing only: 1 + the index of a block of the Poisson solver that never
+                                publishes its border or its progress (FP64 SOR/GS by default or with
+                                sor_blocking 1, Jacobi, mixed), or never arrives at the barriers of
+                                the direct solve in one launch, so that the others' bounded waits run
+                                out (the solve returns CNV_TIMEOUT); 0: off */
     int test_guard_cells;    /* testing only: 1 puts 4 KB of 0xFF bytes (NaN in every lane width)
                                 before and after every field and work buffer and checks them after
                                 each step and Poisson call (CNV_CUDA_ERROR naming the buffer if a

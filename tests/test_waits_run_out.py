@@ -15,6 +15,14 @@ pytestmark = pytest.mark.gpu
 SOLVERS = [
     (64, dict(poisson_type=4)),   # sine transforms in FP64, one launch
     (400, dict(poisson_type=4)),  # in FP32 with corrections, one launch
+    (64, {}),                     # SOR, a cell of each colour per thread: one cluster, mailboxes in shared memory
+    (256, {}),                    # mailboxes in global memory
+    (500, dict(precision=1)),     # FMA
+    (300, dict(poisson_type=1)),  # Gauss-Seidel
+    (600, {}),                    # tiles of many cells
+    (1024, {}),
+    (128, dict(precision=2)),     # mixed: halo cells with their epoch
+    (1500, dict(precision=2)),    # flags
 ]
 
 
