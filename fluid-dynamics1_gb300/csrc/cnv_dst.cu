@@ -21,8 +21,8 @@
 //   - psi is held as 64-bit fixed point: psi = I 2^(E-1023-S) scale / kappa, with E the largest biased exponent
 //     of `in` and S such that the largest |I| is about 2^58. In these units the right-hand side is in * 2^(S-E+1023),
 //     an exponent shift of the double, and the residual in * 2^.. - (a^2 Di + b^2 Dj) I is a sum of 64-bit integers and
-//     the right-hand side's fraction. The integers are taken modulo 2^64, which is exact because the residual itself is small;
-//     the fraction is added to them as a float. (A unit is 2^-58 of the largest |psi|, and psi is up to 0.07 n^2 times the
+//     the right-hand side's fraction. The integers are taken modulo 2^64 (2^128 where a or b is above 512), which is exact
+//     because the residual itself is small; the fraction is added to them as a float. (A unit is 2^-58 of the largest |psi|, and psi is up to 0.07 n^2 times the
 //     right-hand side: without the fraction, cells of one value, all rounded alike, put psi off by 6e-14 at 1000^2, 2e-13 at 2048^2.)
 //   - The first FP32 solve starts from `in`, each later one from the residual, and adds to I. A solve leaves about
 //     3e-7 of the answer, the next 1e-11 .. 1e-10, the third less than the rounding of psi to FP64 for most right-hand sides
@@ -419,12 +419,31 @@ __device__ __forceinline__ double scaled_double(long long v, unsigned long long 
     return scalbn(x, be - 1023);
 }
 
+// scaled_int modulo 2^128.
+__device__ __forceinline__ unsigned __int128 scaled_int128(double x, int E, int S, float& rest) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int f = (int)((b >> 52) & 0x7ff), sh = max(f, 1) - E - 52 + S;
+    const unsigned long long low = scaled_int(x, E, S, rest);
+    if (sh < 10) return (unsigned __int128)(__int128)(long long)low;
+    const unsigned __int128 m = (b & ((1ull << 52) - 1)) | (f ? 1ull << 52 : 0ull);
+    const unsigned __int128 v = sh < 128 ? m << sh : 0;
+    return (long long)b < 0 ? 0 - v : v;
+}
+
 // Conversions between 64-bit integers and floats by 32-bit ones: the instructions on 64-bit types run at the
 // FP64 pipe's rate (two per cycle and SM; the residual of e0 with six of them per cell took 27 us at 1000^2, no more than the later residuals since).
 __device__ __forceinline__ float float_of(unsigned long long v) {
     const unsigned long long a = (long long)v < 0 ? 0ull - v : v;
     const float x = fmaf((float)(unsigned)(a >> 32), 4294967296.f, (float)(unsigned)a);
     return (long long)v < 0 ? -x : x;
+}
+__device__ __forceinline__ float float_of(unsigned __int128 v) {
+    const bool neg = (long long)(v >> 64) < 0;
+    const unsigned __int128 a = neg ? 0 - v : v;
+    const unsigned long long hi = (unsigned long long)(a >> 64), lo = (unsigned long long)a;
+    const float top = fmaf((float)(unsigned)(hi >> 32), 0x1p32f, (float)(unsigned)hi);
+    const float x = fmaf(top, 0x1p64f, fmaf((float)(unsigned)(lo >> 32), 0x1p32f, (float)(unsigned)lo));
+    return neg ? -x : x;
 }
 __device__ __forceinline__ unsigned long long int_of(float v) {  // |v| < 2^50, to nearest
     const int hi = __float2int_rn(v * 0x1p-20f);
@@ -444,6 +463,11 @@ __device__ __forceinline__ unsigned long long fixed_of(float e0, int S) {
 constexpr int kMaxMatrixRadix = 131;  // largest radix whose cosine and sine matrix is tabulated (36 KB)
 constexpr int kOneLaunchRows = 1300;  // largest m whose solve is one launch
 constexpr int kFp64Rows = 304;        // largest m solved in FP64 at once (fp64_radix_ok)
+// Largest extent of the cavity, in lowest terms, whose residual is taken modulo 2^64: it is at most about 2^-22 4 (a^2 + b^2) 2^58 =
+// 2^57. Above (very stretched cells, or extents like 1000 x 999) modulo 2^128, where every pair of ints has room (modelled to 2^31 with
+// exact integers: three solves leave 1e-17 .. 2e-16). us per solve, 64 / 128 bits: 1024^2 229 (511 : 512) / 237 (1000 : 999), 2048^2 1633
+// (1 : 512) / 1700 (1 : 513). Dense products took 4,290 and 29,400 there, FP64 transforms in three launches 610 and 4,370.
+constexpr int kMaxExtent = 512;
 constexpr int kThreads64 = 256;
 constexpr int kThreadsMax = 128;  // threads of a row's (column's) block
 
@@ -509,8 +533,8 @@ __device__ __forceinline__ int fixed_shift(const FftArgs& F, int* s_red) {
     return top ? min(127, 58 - ((top >> 23) - 127)) : 0;
 }
 
-// A: grid row i: the right-hand side or the residual, transformed along j into t.
-template <bool WIDE, bool ONE>
+// A: grid row i: the right-hand side or the residual, transformed along j into t. FAR: the residual modulo 2^128 (kMaxExtent).
+template <bool WIDE, bool ONE, bool FAR>
 __device__ __forceinline__ void pass_a(const FftArgs& F, const Tables<float>& tab, float2* X, int* s_red, int i, int mode, int E,
                                        int S, const double* in) {
     const int N = F.len, ld = F.ld, half = N / 2 + 1, m = F.m;
@@ -551,8 +575,14 @@ __device__ __forceinline__ void pass_a(const FftArgs& F, const Tables<float>& ta
                         h = field<ONE>(p + 1) + field<ONE>(p - 1);
                     }
                     float rest;
-                    const unsigned long long g = scaled_int(row[jj], E, S, rest);
-                    y[q] = float_of(unit ? g - 4 * c + v + h : g - ab * c + a2 * v + b2 * h) + rest;
+                    if constexpr (FAR) {
+                        auto wide = [](unsigned long long x) { return (unsigned __int128)(__int128)(long long)x; };
+                        const unsigned __int128 a = a2, b = b2, g = scaled_int128(row[jj], E, S, rest);
+                        y[q] = float_of(g - 2 * (a + b) * wide(c) + a * wide(v) + b * wide(h)) + rest;
+                    } else {
+                        const unsigned long long g = scaled_int(row[jj], E, S, rest);
+                        y[q] = float_of(unit ? g - 4 * c + v + h : g - ab * c + a2 * v + b2 * h) + rest;
+                    }
                 }
             }
             put_z<1, float>(F, tab, X, j, 0, y[0], y[1]);
@@ -673,7 +703,7 @@ __device__ __forceinline__ int c_mode(int k, int solves) {
 }
 
 // The passes as launches of their own: solve k of `solves`, a row (cols_b columns) per block.
-template <int FORM>
+template <int FORM, bool FAR>
 __global__ void __launch_bounds__(kThreadsMax, blocks_per_sm(FORM)) k_dst_a(FftArgs F, int k, const double* in) {
     extern __shared__ float2 fsm[];
     __shared__ int s_red[8];
@@ -681,7 +711,7 @@ __global__ void __launch_bounds__(kThreadsMax, blocks_per_sm(FORM)) k_dst_a(FftA
     const int E = k ? F.ctl[0] : 0;
     const int S = k == 0 ? 0 : k == 1 ? fixed_shift<false>(F, s_red) : F.ctl[1];
     if (k == 1 && blockIdx.x == 0 && threadIdx.x == 0) F.ctl[1] = S;
-    pass_a<FORM == kWide, false>(F, tab, fsm, s_red, 1 + blockIdx.x, a_mode(k), E, S, in);
+    pass_a<FORM == kWide, false, FAR>(F, tab, fsm, s_red, 1 + blockIdx.x, a_mode(k), E, S, in);
 }
 
 template <int RP, int FORM>
@@ -729,7 +759,7 @@ struct GridBarrier {
 };
 
 // All passes of a solve in one cooperative launch, block b taking row b + 1 and column b + 1, with a grid barrier between passes.
-template <int FORM>
+template <int FORM, bool FAR>
 __global__ void __launch_bounds__(kThreadsMax, blocks_per_sm(FORM))
     k_dst_all(FftArgs F, int solves, const double* in, KScale ks, DstDest dst, Ctrl* ctrl, long long timeout_ns, int stall_block) {
     extern __shared__ float2 fsm[];
@@ -741,7 +771,7 @@ __global__ void __launch_bounds__(kThreadsMax, blocks_per_sm(FORM))
     int E = 0, S = 0;
     for (int k = 0; k < solves; ++k) {
         if (k == 1) S = fixed_shift<true>(F, s_red);
-        pass_a<FORM == kWide, true>(F, tab, fsm, s_red, i, a_mode(k), E, S, in);
+        pass_a<FORM == kWide, true, FAR>(F, tab, fsm, s_red, i, a_mode(k), E, S, in);
         if (!bar.wait()) return;
         if (k == 0) E = exponent<true>(F, s_red);
         pass_b<1, FORM == kWide, true>(F, tab, fsm, i, k == 0, E);
@@ -931,6 +961,13 @@ cudaError_t launch_pass(void (*k)(Params...), int blocks, int threads, int smem,
     return cudaLaunchKernelEx(&cfg, k, Params(args)...);
 }
 
+template <bool FAR>
+auto kernel_a(int form) { return form == kSmall ? k_dst_a<kSmall, FAR> : form == kMid ? k_dst_a<kMid, FAR> : k_dst_a<kWide, FAR>; }
+template <bool FAR>
+auto kernel_all(int form) { return form == kSmall ? k_dst_all<kSmall, FAR> : form == kMid ? k_dst_all<kMid, FAR> : k_dst_all<kWide, FAR>; }
+auto kernel_a(int form, bool far) { return far ? kernel_a<true>(form) : kernel_a<false>(form); }
+auto kernel_all(int form, bool far) { return far ? kernel_all<true>(form) : kernel_all<false>(form); }
+
 cudaError_t solve(const DstPlan& P, const double* in, double scale, const DstDest& d, cudaStream_t s) {
     const int m = P.m;
     cudaError_t e;
@@ -941,11 +978,10 @@ cudaError_t solve(const DstPlan& P, const double* in, double scale, const DstDes
         if (P.fp64)
             return launch_pass(k_dst_fp64, m, kThreads64, P.smem_a, true, s, F, in, scale, d, P.ctrl, P.timeout_ns, P.stall_block);
         if (P.one_launch) {
-            const auto k1 = P.form == kSmall ? k_dst_all<kSmall> : P.form == kMid ? k_dst_all<kMid> : k_dst_all<kWide>;
-            return launch_pass(k1, m, P.threads_a, P.smem_a, true, s, F, P.solves, in, ks, d, P.ctrl, P.timeout_ns, P.stall_block);
+            return launch_pass(kernel_all(P.form, P.far), m, P.threads_a, P.smem_a, true, s, F, P.solves, in, ks, d, P.ctrl, P.timeout_ns, P.stall_block);
         }
         for (int k = 0; k < P.solves; ++k) {
-            const auto ka = P.form == kSmall ? k_dst_a<kSmall> : P.form == kMid ? k_dst_a<kMid> : k_dst_a<kWide>;
+            const auto ka = kernel_a(P.form, P.far);
             const auto kb = F.cols_b == 2 ? (P.form == kMid ? k_dst_b<2, kMid> : k_dst_b<2, kWide>)
                                           : (P.form == kSmall ? k_dst_b<1, kSmall> : P.form == kMid ? k_dst_b<1, kMid> : k_dst_b<1, kWide>);
             const auto kc = P.form == kSmall ? k_dst_c<kSmall> : P.form == kMid ? k_dst_c<kMid> : k_dst_c<kWide>;
@@ -1035,7 +1071,7 @@ template <class R>
 bool plan_fft(DstPlan* P, int a, int b, int sms, int smem_max, const Ctrl* ctrl, int* status) {
     const int m = P->m, len = m + 1;
     std::vector<int> rad;
-    if (a > 512 || b > 512 || !radices(len, &rad)) return false;
+    if (!radices(len, &rad)) return false;
     FftArgs& F = P->F;
     int ncs = 0, ncm = 0;  // entries of the radices' tables and of the large ones' matrices
     for (int p : rad) {
@@ -1157,11 +1193,12 @@ bool plan_fft(DstPlan* P, int a, int b, int sms, int smem_max, const Ctrl* ctrl,
     P->solves = solves_needed(len, rad[0], (double)F.a2, (double)F.b2);
     P->kappa = 0.5 * (P->dy2 / F.a2 + P->dx2 / F.b2);
     // the same limit for every plan: a function's attribute is shared by all of them
-    const void* small[] = {(const void*)k_dst_a<kSmall>, (const void*)k_dst_b<1, kSmall>, (const void*)k_dst_c<kSmall>, (const void*)k_dst_all<kSmall>};
-    const void* mid[] = {(const void*)k_dst_a<kMid>, F.cols_b == 2 ? (const void*)k_dst_b<2, kMid> : (const void*)k_dst_b<1, kMid>,
-                         (const void*)k_dst_c<kMid>, (const void*)k_dst_all<kMid>};
-    const void* wide[] = {(const void*)k_dst_a<kWide>, F.cols_b == 2 ? (const void*)k_dst_b<2, kWide> : (const void*)k_dst_b<1, kWide>,
-                          (const void*)k_dst_c<kWide>, (const void*)k_dst_all<kWide>};
+    P->far = std::max(a, b) > kMaxExtent;
+    const void* ka = (const void*)kernel_a(P->form, P->far);
+    const void* kall = (const void*)kernel_all(P->form, P->far);
+    const void* small[] = {ka, (const void*)k_dst_b<1, kSmall>, (const void*)k_dst_c<kSmall>, kall};
+    const void* mid[] = {ka, F.cols_b == 2 ? (const void*)k_dst_b<2, kMid> : (const void*)k_dst_b<1, kMid>, (const void*)k_dst_c<kMid>, kall};
+    const void* wide[] = {ka, F.cols_b == 2 ? (const void*)k_dst_b<2, kWide> : (const void*)k_dst_b<1, kWide>, (const void*)k_dst_c<kWide>, kall};
     const void* fp64[] = {(const void*)k_dst_fp64, nullptr, nullptr, nullptr};
     const void* const* kernels = kF64 ? fp64 : P->form == kSmall ? small : P->form == kMid ? mid : wide;
     for (int k = 0; k < 4 && kernels[k]; ++k)

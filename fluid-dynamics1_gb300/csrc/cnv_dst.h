@@ -52,6 +52,7 @@ struct DstPlan {
     int form = 0;              // the passes' form (cnv_dst.cu)
     bool one_launch = false;   // all passes in one cooperative launch, whose waits report to ctrl
     bool fp64 = false;         // in FP64 at once (small grids)
+    bool far = false;          // residual modulo 2^128 (very stretched cells)
     Ctrl* ctrl = nullptr;
     long long timeout_ns = 0;
     int stall_block = -1;      // testing only: a block of the one-launch forms that never arrives at their barriers
