@@ -106,6 +106,11 @@ struct BatchLaunch {
 namespace {
 
 constexpr int kMaxBatchThreads = 1024;
+// A batch of cavities smaller than this runs k_batch<SMALL>: scalar sweeps, FP64 multiplications in the passes. With a cell a thread
+// at most a step is a chain of latencies, which the vector sweeps' set-up and the integer multiplications lengthen (a kernel of its own:
+// a second copy of the step in one kernel cost the larger cavities 2 %). us per step, k_batch<false> / k_batch<true>: 8^2 203 / 180, 16^2
+// 203 / 188, 22^2 237 / 226, 24^2 236 / 245, 64^2 532 / 750.
+constexpr int kSmallN = 24;
 
 // The dynamic shared memory of k_batch; the sweeps address it through this array with integer offsets, so every access
 // compiles to a shared-memory load or store.
@@ -257,7 +262,9 @@ __device__ void batch_half_sweep(float* __restrict__ ec, const float* __restrict
 }
 
 // One time step of one cavity by the whole block. Returns the step's status.
+template <bool SMALL>
 __device__ int batch_step(CavityDesc& C, float* smem, int max_outer, double rtol, bool warm, double* s_red) {
+    constexpr int MUL = SMALL ? kMulFp64 : kMulInt;
     const int n = C.n, P = C.pitch;
     const int tid = threadIdx.x, nt = blockDim.x;
     double* w_in = C.w[C.cur];
@@ -272,15 +279,15 @@ __device__ int batch_step(CavityDesc& C, float* smem, int max_outer, double rtol
         const int j = side == 2 ? 0 : side == 3 ? n - 1 : t;
         auto U = [&](int r, int cc) { return vel_bc(C.u, n, r, cc, bc.u1, bc.u2, bc.u3, bc.u4); };
         auto V = [&](int r, int cc) { return vel_bc(C.v, n, r, cc, bc.v1, bc.v2, bc.v3, bc.v4); };
-        w_in[(size_t)i * n + j] = dsub(along_j<kMulInt>(B->d1x, n, i, j, V), along_i<kMulInt>(B->d1y, n, i, j, U));
+        w_in[(size_t)i * n + j] = dsub(along_j<MUL>(B->d1x, n, i, j, V), along_i<MUL>(B->d1y, n, i, j, U));
     }
     __syncthreads();
     // transport: derivatives of w and the Euler update (src/fluiddyn.c:98); g = c4 * (-w)
     for (int k = tid; k < n * n; k += nt) {
         const int i = k / n, j = k - (k / n) * n;
         auto W = [&](int r, int cc) { return w_in[(size_t)r * n + cc]; };
-        const double wx = along_j<kMulInt>(B->d1x, n, i, j, W), wy = along_i<kMulInt>(B->d1y, n, i, j, W);
-        const double wxx = along_j<kMulInt>(B->d2x, n, i, j, W), wyy = along_i<kMulInt>(B->d2y, n, i, j, W);
+        const double wx = along_j<MUL>(B->d1x, n, i, j, W), wy = along_i<MUL>(B->d1y, n, i, j, W);
+        const double wxx = along_j<MUL>(B->d2x, n, i, j, W), wyy = along_i<MUL>(B->d2y, n, i, j, W);
         const double ue = vel_bc(C.u, n, i, j, bc.u1, bc.u2, bc.u3, bc.u4);
         const double ve = vel_bc(C.v, n, i, j, bc.v1, bc.v2, bc.v3, bc.v4);
         const double conv = dsub(dmul(-ue, wx), dmul(ve, wy));
@@ -304,10 +311,13 @@ __device__ int batch_step(CavityDesc& C, float* smem, int max_outer, double rtol
     float* rqc[2] = {C.smem_mode == 2 ? rq_s[0] : C.rq[0], C.smem_mode == 2 ? rq_s[1] : C.rq[1]};
     const int rp = C.smem_mode == 2 ? sp : P;
     const float wxf = (float)(C.dx2 / C.den), wyf = (float)(C.dy2 / C.den), betaf = (float)C.beta;
-    const QuadSweep Q = quad_sweep(n, n - 2, wxf, wyf, betaf);
-    if (C.vec && C.smem_mode == 2)  // R/den is 0 on the walls and in the padding
-        for (int k = tid; k < 2 * eplane; k += nt) rq_s[0][k] = 0.0f;
-    __syncthreads();
+    QuadSweep Q;
+    if constexpr (!SMALL) {
+        Q = quad_sweep(n, n - 2, wxf, wyf, betaf);
+        if (C.vec && C.smem_mode == 2)  // R/den is 0 on the walls and in the padding
+            for (int k = tid; k < 2 * eplane; k += nt) rq_s[0][k] = 0.0f;
+        __syncthreads();
+    }
     double rel = 0.0, gnorm = 0.0;
     int outer = 0, status = CNV_NOT_CONVERGED;
     long long sweeps = 0;
@@ -338,9 +348,9 @@ __device__ int batch_step(CavityDesc& C, float* smem, int max_outer, double rtol
         __syncthreads();
         for (int s = 0; s < 2 * C.inner; ++s) {
             const int c = s & 1;
-            if (C.vec && C.smem_mode == 2)
+            if (!SMALL && C.vec && C.smem_mode == 2)
                 quad_half_sweep<kRhsShared>(Q, c * eplane, (c ^ 1) * eplane, nullptr, (2 + c) * eplane, ep, 0, 1, n - 1, c);
-            else if (C.vec)
+            else if (!SMALL && C.vec)
                 quad_half_sweep<kRhsOwn>(Q, c * eplane, (c ^ 1) * eplane, rqc[c], 0, ep, rp, 1, n - 1, c);
             else batch_half_sweep(ec[c], ec[c ^ 1], rqc[c], n, ep, rp, c, wxf, wyf, betaf);
             __syncthreads();
@@ -360,8 +370,8 @@ __device__ int batch_step(CavityDesc& C, float* smem, int max_outer, double rtol
     auto PS = [&](int y, int x) { return C.psi[(y + x) & 1][(size_t)y * P + (x >> 1)]; };
     for (int k = tid; k < n * n; k += nt) {
         const int i = k / n, j = k - (k / n) * n;
-        C.u[k] = along_i<kMulInt>(B->d1y, n, i, j, PS);
-        C.v[k] = -along_j<kMulInt>(B->d1x, n, i, j, PS);
+        C.u[k] = along_i<MUL>(B->d1y, n, i, j, PS);
+        C.v[k] = -along_j<MUL>(B->d1x, n, i, j, PS);
         C.psi_rm[k] = PS(i, j);
     }
     __syncthreads();
@@ -371,7 +381,7 @@ __device__ int batch_step(CavityDesc& C, float* smem, int max_outer, double rtol
     auto Vf = [&](int r, int cc) { return C.v[(size_t)r * n + cc]; };
     for (int k = tid; k < n * n; k += nt) {
         const int i = k / n, j = k - (k / n) * n;
-        const double cv = dadd(along_j<kMulInt>(B->d1x, n, i, j, Uf), along_i<kMulInt>(B->d1y, n, i, j, Vf));
+        const double cv = dadd(along_j<MUL>(B->d1x, n, i, j, Uf), along_i<MUL>(B->d1y, n, i, j, Vf));
         mx = cv > mx ? cv : mx;
         mn = cv < mn ? cv : mn;
     }
@@ -392,6 +402,7 @@ __device__ int batch_step(CavityDesc& C, float* smem, int max_outer, double rtol
 // ------------------------------------------------------------------------------ group jobs
 constexpr int kStripSweeps = 4;                // FP32 sweeps between border exchanges (8: 1 % faster, more smem)
 constexpr int kStripHalo = 2 * kStripSweeps;   // halo rows of a strip
+static_assert(kSmallN <= 4 * kStripHalo, "k_batch<SMALL> has no strips");
 
 // Barrier of the g blocks of a group (counter gs->bar, target gen). False if the wait gave up
 // (2 s; sets *abort = CNV_TIMEOUT) or another block has aborted; the caller leaves the job.
@@ -653,6 +664,7 @@ __device__ int group_step(CavityDesc& C, int cur, int r, int g, float* smem, int
     return status;
 }
 
+template <bool SMALL>
 __global__ void __launch_bounds__(kMaxBatchThreads) k_batch(BatchLaunch L) {
     float* const smem = bt_smem;
     __shared__ double s_red[64];
@@ -661,14 +673,14 @@ __global__ void __launch_bounds__(kMaxBatchThreads) k_batch(BatchLaunch L) {
     for (int e = L.sched_off[blockIdx.x]; e < L.sched_off[blockIdx.x + 1]; ++e) {
         const SchedEntry J = L.sched[e];
         CavityDesc& C = L.cav[J.cav];
-        if (J.group == 1) {
+        if (SMALL || J.group == 1) {
             if (threadIdx.x == 0) {
                 C.sweeps = 0;
                 C.steps_done = 0;
             }
             __syncthreads();
             for (int t = 0; t < nsteps; ++t) {
-                const int st = batch_step(C, smem, L.max_outer, L.rtol, L.warm != 0, s_red);
+                const int st = batch_step<SMALL>(C, smem, L.max_outer, L.rtol, L.warm != 0, s_red);
                 if (threadIdx.x == 0) C.steps_done = t + 1;
                 if (st != CNV_OK) break;
             }
@@ -823,6 +835,14 @@ double step_cost(int n, int g, int smem_mode) {
     return (4.0 * n * cells / rate * halo + 0.061 * cells) / g + barriers;
 }
 
+bool small_batch(const cnv_batch* b) {
+    return std::all_of(b->host_desc.begin(), b->host_desc.end(), [](const CavityDesc& d) { return d.n < kSmallN; });
+}
+
+const void* kernel_of(const cnv_batch* b) {
+    return small_batch(b) ? reinterpret_cast<const void*>(&k_batch<true>) : reinterpret_cast<const void*>(&k_batch<false>);
+}
+
 int build_graph(cnv_batch* b) {
     if (b->graph) {
         cudaGraphExecDestroy(b->graph);
@@ -840,7 +860,8 @@ int build_graph(cnv_batch* b) {
     L.rtol = b->rtol;
     L.warm = b->warm;
     L.smem_floats = b->smem_bytes / 4;
-    BCUDA(cudaFuncSetAttribute(k_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, b->smem_bytes));
+    const void* kernel = kernel_of(b);
+    BCUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, b->smem_bytes));
     cudaGraph_t g = nullptr;
     BCUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t me = cudaMemsetAsync(b->gsync, 0, sizeof(GroupSync) * b->count, b->stream);
@@ -858,7 +879,7 @@ int build_graph(cnv_batch* b) {
     cfg.numAttrs = 1;
     void* args[] = {&L};
     const cudaError_t le =
-        me != cudaSuccess ? me : cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(&k_batch), args);
+        me != cudaSuccess ? me : cudaLaunchKernelExC(&cfg, kernel, args);
     cudaError_t e = cudaStreamEndCapture(b->stream, &g);
     if (le != cudaSuccess) {
         if (g) cudaGraphDestroy(g);
@@ -1011,17 +1032,19 @@ int set_shape(cnv_batch* b, int threads, int per_sm) {
     b->threads = threads;
     b->smem_bytes = std::min(optin, dev_smem / per_sm - 2048) & ~255;
     int occ = 0;
-    BCUDA(cudaFuncSetAttribute(k_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, b->smem_bytes));
-    BCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_batch, threads, b->smem_bytes));
+    const void* kernel = kernel_of(b);
+    BCUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, b->smem_bytes));
+    BCUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, threads, b->smem_bytes));
     if (occ < 1) return bfail(CNV_CUDA_ERROR, "batched kernel does not fit on an SM");
     b->blocks = std::min(occ, per_sm) * b->sms;
     // per-cavity placement of the FP32 correction for this shared-memory size, and row strips
     assign_groups(b->host_desc, b->smem_bytes, b->split, b->split_min_n, b->group_by_n);
     // the vector sweeps where the tile fits with rows of whole vectors (nearly always: the plan counts one column more)
+    const bool small = small_batch(b);
     for (auto& d : b->host_desc) {
         const int p4 = ((d.n + 1) / 2 + 3) / 4 * 4;
         const size_t rows = d.group > 1 ? (size_t)(d.n + d.group - 1) / d.group + 2 * kStripHalo : d.n;
-        d.vec = d.smem_mode >= 1 && 8 * rows * p4 <= (size_t)b->smem_bytes ? 1 : 0;
+        d.vec = !small && d.smem_mode >= 1 && 8 * rows * p4 <= (size_t)b->smem_bytes ? 1 : 0;
         d.epitch = d.vec ? p4 : d.spitch;
         if (d.vec && d.smem_mode == 2 && 16 * rows * p4 > (size_t)b->smem_bytes) d.smem_mode = 1;
     }
