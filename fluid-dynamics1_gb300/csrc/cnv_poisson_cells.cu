@@ -1,5 +1,5 @@
 // cnv_poisson_cells.cu -- FP64 red-black SOR / Gauss-Seidel up to 1100^2: a cell of each colour per thread (k_poisson_cells, to
-// 530^2), or tiles of many cells in shared memory (k_poisson_rows, described there).
+// 515^2; FMA 514^2), or tiles of many cells in shared memory (k_poisson_rows, described there).
 //
 // The same solve as cnv_poisson.cu (the reference's point update and its stop rule, bit for bit), for grids where a sweep
 // is a chain of latencies: 64^2 took 5.9 us per sweep and 256^2 6.2 with shared-memory tiles and a border exchange per four
@@ -47,7 +47,10 @@ constexpr int kHist = 8;       // sweeps kept in shared memory
 constexpr int kLag = 6;        // a sweep starts when the one kLag before it is known not to have converged
 static_assert(kHist > kLag, "the iterate that converged is still in the ring");
 constexpr int kNormRing = 32;  // sweeps' norms in flight: at least 3 kLag (see check_norms)
-constexpr int kMinNormWarps = 2, kMaxNormWarps = 6;  // a whole sweep's share each, in turn
+// Norm warps, a whole sweep's share each, in turn: at most 6, and a tile that leaves room for fewer than 3 (FMA, whose sweeps are
+// shorter: 4) is left to k_poisson_rows, because their pace is then the sweep's. us per sweep with 4 / 3 / 2 of them, k_poisson_rows: general SOR
+// 514^2 6.6, 515^2 7.5, 516^2 10.9 against 8.5 .. 8.6; FMA 4.8, 6.6, 10.5 against 5.6.
+constexpr int kMinNormWarps = 3, kMinNormWarpsFma = 4, kMaxNormWarps = 6;
 
 // The norm's ring. A slot's words: the chunk sums of e_k for the k of that slot, all turns of the ring added up, over the blocks
 // b with b % kParts = part. Above kCountBit each word counts the blocks that added (a turn's sums stay below 2^50: 19 blocks of
@@ -891,7 +894,7 @@ cudaLaunchConfig_t cells_config(const CellsPlan& P, cudaLaunchAttribute* attr, c
 }
 
 // Tiles, threads and mailbox length of a gx x gy cut; false where a tile is a single row or column.
-bool cells_cut(int n, int gx, int gy, CellsPlan* P) {
+bool cells_cut(int n, int gx, int gy, int min_norm_warps, CellsPlan* P) {
     P->gx = gx;
     P->gy = gy;
     const int ni = n - 2, W = (ni + gx - 1) / gx, H = (ni + gy - 1) / gy;  // of the largest tile
@@ -900,7 +903,7 @@ bool cells_cut(int n, int gx, int gy, CellsPlan* P) {
     P->side = std::max(W, H);
     P->tc = colour_threads(W, H);
     P->tc = (P->tc + 31) / 32 * 32;
-    P->norm_warps = std::max(kMinNormWarps, std::min(kMaxNormWarps, 31 - P->tc / 32));
+    P->norm_warps = std::max(min_norm_warps, std::min(kMaxNormWarps, 31 - P->tc / 32));
     P->threads = P->tc + 32 * (P->norm_warps + 1);  // and the verdict's warp
     return true;
 }
@@ -912,19 +915,19 @@ CellsPlan cells_plan(int n, int sms, size_t smem_max, Arith a, int kind, bool fo
     const CellsPlan none{};
     CellsPlan best{}, q{};
     if (kind != CNV_POISSON_SOR && kind != CNV_POISSON_GS) return none;
-    const int cap = std::min(sms, kMaxSolverBlocks);
+    const int cap = std::min(sms, kMaxSolverBlocks), min_norm = a == Arith::kFma ? kMinNormWarpsFma : kMinNormWarps;
     // One cluster up to 90^2 (the exact arithmetic) or 112^2 (FMA, with fewer FP64 operations a cell): its 16 SMs' FP64 pipes
     // take as long there as the hops between all SMs (general SOR: 64^2 1.76 us a sweep against 2.61, 97^2 2.91 against 2.65;
     // FMA: 112^2 1.90 against 1.98).
     if (n <= (a == Arith::kFma ? 112 : 90)) {
         const int g = std::min(kClusterSide, (n - 2) / 2);
-        if (g < 1 || !cells_cut(n, g, g, &best)) return none;
+        if (g < 1 || !cells_cut(n, g, g, min_norm, &best)) return none;
         best.cluster = 1;
         if (best.threads > 640) return none;
     } else {
         for (int gx = 1; gx <= cap; ++gx)
             for (int gy = cap / gx; gy >= 1 && gy >= cap / gx - 1; --gy)
-                if (cells_cut(n, gx, gy, &q) && q.threads <= 1024 &&
+                if (cells_cut(n, gx, gy, min_norm, &q) && q.threads <= 1024 &&
                     (best.tc == 0 || q.tc < best.tc || (q.tc == best.tc && q.side < best.side)))
                     best = q;
         if (best.tc == 0 && n <= kRowsMax) {
@@ -933,7 +936,7 @@ CellsPlan cells_plan(int n, int sms, size_t smem_max, Arith a, int kind, bool fo
             const int ni = n - 2;
             for (int gx = 1; gx <= cap; ++gx) {
                 const int gy = cap / gx, W = (ni + gx - 1) / gx, H = (ni + gy - 1) / gy;
-                if (!cells_cut(n, gx, gy, &q) || ni / gx < 3 || ni / gy < 3) continue;
+                if (!cells_cut(n, gx, gy, min_norm, &q) || ni / gx < 3 || ni / gy < 3) continue;
                 const int cost = W * H + W + H, nq = (W - 1) / 2, ne = edge_cells(W, H);
                 if (best.tc && cost >= cells) continue;
                 // fewer threads with more registers unless that costs a turn of the rows; warps of their own for the edge, or inner
