@@ -158,10 +158,11 @@ __device__ __noinline__ void mixed_half_sweep(int sc_off, int so_off, int rq_off
 
 // FP64 residual R = g - A psi on the block's own cells, its norm's (and in outer iteration 0 |g|'s) partial sums, and
 // the FP32 right-hand side R/den of the correction: cell (i, j) of colour c at rq[c][i * pitch + ((j - first) >> 1)].
-template <int FIRST>
+// WARPS: the block's warps (0: blockDim.x / 32), so that the last sum's loads are issued together.
+template <int FIRST, int WARPS>
 __device__ __forceinline__ void mixed_residual(const MixedLaunch& L, const MTile& t, MixedSync* sy, int outer,
                                                double (*s_red)[2]) {
-    const int P = L.pitch, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int P = L.pitch, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = WARPS ? WARPS : blockDim.x >> 5;
     const double dx2 = L.dx2, dy2 = L.dy2, den = L.den;
     double rr = 0.0, gg = 0.0;
     for (int i = t.r0 + warp; i < t.r1; i += warps) {
@@ -288,7 +289,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_mixed(MixedLaunch L) {
     double rel = 0.0;
 
     for (outer = 0;; ++outer) {
-        mixed_residual<0>(L, t, sy, outer, s_red);
+        mixed_residual<0, kWarps>(L, t, sy, outer, s_red);
         if (!grid_sync(sy, bar, ctl, L.timeout_ns, &s_ok)) { status = CNV_TIMEOUT; break; }
         rel = mixed_norm(sy, s_tot);
         if (!isfinite(rel)) { status = CNV_NONFINITE; break; }
@@ -627,7 +628,7 @@ __global__ void __launch_bounds__(MAXT, 1) k_mixed_reg(MixedLaunch L) {
     long long sweeps = 0;
     double rel = 0.0;
     for (outer = 0;; ++outer) {
-        mixed_residual<1>(L, t, sy, outer, s_red);
+        mixed_residual<1, 0>(L, t, sy, outer, s_red);
         if (!grid_sync(sy, bar, ctl, L.timeout_ns, &s_ok)) { status = CNV_TIMEOUT; break; }
         rel = mixed_norm(sy, s_tot);
         if (!isfinite(rel)) { status = CNV_NONFINITE; break; }
