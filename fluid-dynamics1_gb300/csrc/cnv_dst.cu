@@ -702,12 +702,12 @@ __device__ __forceinline__ int c_mode(int k, int solves) {
     return k == 0 ? kToE0 : k == solves - 1 ? kAddLast : k == 1 ? kAddToE0 : kAdd;
 }
 
-// The passes as launches of their own: solve k of `solves`, a row (cols_b columns) per block.
+// The passes as launches of their own (kMid and kWide): solve k of `solves`, a row (cols_b columns) per block.
 template <int FORM, bool FAR>
 __global__ void __launch_bounds__(kThreadsMax, blocks_per_sm(FORM)) k_dst_a(FftArgs F, int k, const double* in) {
     extern __shared__ float2 fsm[];
     __shared__ int s_red[8];
-    const Tables<float> tab = begin_pass<float, FORM == kSmall>(F, reinterpret_cast<float4*>(fsm + F.fields));
+    const Tables<float> tab = begin_pass<float, false>(F, reinterpret_cast<float4*>(fsm + F.fields));
     const int E = k ? F.ctl[0] : 0;
     const int S = k == 0 ? 0 : k == 1 ? fixed_shift<false>(F, s_red) : F.ctl[1];
     if (k == 1 && blockIdx.x == 0 && threadIdx.x == 0) F.ctl[1] = S;
@@ -718,7 +718,7 @@ template <int RP, int FORM>
 __global__ void __launch_bounds__(RP * kThreadsMax, blocks_per_sm(FORM) / RP) k_dst_b(FftArgs F, int k) {
     extern __shared__ float2 fsm[];
     __shared__ int s_red[8];
-    const Tables<float> tab = begin_pass<float, FORM == kSmall>(F, reinterpret_cast<float4*>(fsm + F.fields * RP));
+    const Tables<float> tab = begin_pass<float, false>(F, reinterpret_cast<float4*>(fsm + F.fields * RP));
     const int E = k ? 0 : exponent<false>(F, s_red);
     if (k == 0 && blockIdx.x == 0 && threadIdx.x == 0) F.ctl[0] = E;
     pass_b<RP, FORM == kWide, false>(F, tab, fsm, blockIdx.x * RP, k == 0, E);
@@ -728,7 +728,7 @@ template <int FORM>
 __global__ void __launch_bounds__(kThreadsMax, blocks_per_sm(FORM)) k_dst_c(FftArgs F, int k, int solves, KScale ks, DstDest dst) {
     extern __shared__ float2 fsm[];
     __shared__ int s_red[8];
-    const Tables<float> tab = begin_pass<float, FORM == kSmall>(F, reinterpret_cast<float4*>(fsm + F.fields));
+    const Tables<float> tab = begin_pass<float, false>(F, reinterpret_cast<float4*>(fsm + F.fields));
     pass_c<FORM == kWide, false>(F, tab, fsm, s_red, 1 + blockIdx.x, c_mode(k, solves), F.ctl[0], k ? F.ctl[1] : 0, ks, dst);
 }
 
@@ -961,12 +961,15 @@ cudaError_t launch_pass(void (*k)(Params...), int blocks, int threads, int smem,
     return cudaLaunchKernelEx(&cfg, k, Params(args)...);
 }
 
-template <bool FAR>
-auto kernel_a(int form) { return form == kSmall ? k_dst_a<kSmall, FAR> : form == kMid ? k_dst_a<kMid, FAR> : k_dst_a<kWide, FAR>; }
+// The kernels of a plan. k_dst_a, k_dst_b and k_dst_c come in the forms that may need more than one launch (plan_fft).
 template <bool FAR>
 auto kernel_all(int form) { return form == kSmall ? k_dst_all<kSmall, FAR> : form == kMid ? k_dst_all<kMid, FAR> : k_dst_all<kWide, FAR>; }
-auto kernel_a(int form, bool far) { return far ? kernel_a<true>(form) : kernel_a<false>(form); }
-auto kernel_all(int form, bool far) { return far ? kernel_all<true>(form) : kernel_all<false>(form); }
+auto kernel_all(const DstPlan& P) { return P.far ? kernel_all<true>(P.form) : kernel_all<false>(P.form); }
+auto kernel_a(const DstPlan& P) {
+    return P.form == kMid ? (P.far ? k_dst_a<kMid, true> : k_dst_a<kMid, false>) : P.far ? k_dst_a<kWide, true> : k_dst_a<kWide, false>;
+}
+auto kernel_b(const DstPlan& P) { return P.F.cols_b == 1 ? k_dst_b<1, kWide> : P.form == kMid ? k_dst_b<2, kMid> : k_dst_b<2, kWide>; }
+auto kernel_c(const DstPlan& P) { return P.form == kMid ? k_dst_c<kMid> : k_dst_c<kWide>; }
 
 cudaError_t solve(const DstPlan& P, const double* in, double scale, const DstDest& d, cudaStream_t s) {
     const int m = P.m;
@@ -978,16 +981,12 @@ cudaError_t solve(const DstPlan& P, const double* in, double scale, const DstDes
         if (P.fp64)
             return launch_pass(k_dst_fp64, m, kThreads64, P.smem_a, true, s, F, in, scale, d, P.ctrl, P.timeout_ns, P.stall_block);
         if (P.one_launch) {
-            return launch_pass(kernel_all(P.form, P.far), m, P.threads_a, P.smem_a, true, s, F, P.solves, in, ks, d, P.ctrl, P.timeout_ns, P.stall_block);
+            return launch_pass(kernel_all(P), m, P.threads_a, P.smem_a, true, s, F, P.solves, in, ks, d, P.ctrl, P.timeout_ns, P.stall_block);
         }
         for (int k = 0; k < P.solves; ++k) {
-            const auto ka = kernel_a(P.form, P.far);
-            const auto kb = F.cols_b == 2 ? (P.form == kMid ? k_dst_b<2, kMid> : k_dst_b<2, kWide>)
-                                          : (P.form == kSmall ? k_dst_b<1, kSmall> : P.form == kMid ? k_dst_b<1, kMid> : k_dst_b<1, kWide>);
-            const auto kc = P.form == kSmall ? k_dst_c<kSmall> : P.form == kMid ? k_dst_c<kMid> : k_dst_c<kWide>;
-            if ((e = launch_pass(ka, m, P.threads_a, P.smem_a, false, s, F, k, in)) != cudaSuccess) return e;
-            if ((e = launch_pass(kb, blocks_b, P.threads_b, P.smem_b, false, s, F, k)) != cudaSuccess) return e;
-            if ((e = launch_pass(kc, m, P.threads_a, P.smem_a, false, s, F, k, P.solves, ks, d)) != cudaSuccess) return e;
+            if ((e = launch_pass(kernel_a(P), m, P.threads_a, P.smem_a, false, s, F, k, in)) != cudaSuccess) return e;
+            if ((e = launch_pass(kernel_b(P), blocks_b, P.threads_b, P.smem_b, false, s, F, k)) != cudaSuccess) return e;
+            if ((e = launch_pass(kernel_c(P), m, P.threads_a, P.smem_a, false, s, F, k, P.solves, ks, d)) != cudaSuccess) return e;
         }
         return cudaSuccess;
     }
@@ -1068,7 +1067,7 @@ struct Roots {
 
 // The FFT path's tables and fields for len = m + 1; false where it does not apply.
 template <class R>
-bool plan_fft(DstPlan* P, int a, int b, int sms, int smem_max, const Ctrl* ctrl, int* status) {
+bool plan_fft(DstPlan* P, int a, int b, int sms, int smem_max, int* status) {
     const int m = P->m, len = m + 1;
     std::vector<int> rad;
     if (!radices(len, &rad)) return false;
@@ -1192,24 +1191,23 @@ bool plan_fft(DstPlan* P, int a, int b, int sms, int smem_max, const Ctrl* ctrl,
     F.len = len;
     P->solves = solves_needed(len, rad[0], (double)F.a2, (double)F.b2);
     P->kappa = 0.5 * (P->dy2 / F.a2 + P->dx2 / F.b2);
-    // the same limit for every plan: a function's attribute is shared by all of them
     P->far = std::max(a, b) > kMaxExtent;
-    const void* ka = (const void*)kernel_a(P->form, P->far);
-    const void* kall = (const void*)kernel_all(P->form, P->far);
-    const void* small[] = {ka, (const void*)k_dst_b<1, kSmall>, (const void*)k_dst_c<kSmall>, kall};
-    const void* mid[] = {ka, F.cols_b == 2 ? (const void*)k_dst_b<2, kMid> : (const void*)k_dst_b<1, kMid>, (const void*)k_dst_c<kMid>, kall};
-    const void* wide[] = {ka, F.cols_b == 2 ? (const void*)k_dst_b<2, kWide> : (const void*)k_dst_b<1, kWide>, (const void*)k_dst_c<kWide>, kall};
-    const void* fp64[] = {(const void*)k_dst_fp64, nullptr, nullptr, nullptr};
-    const void* const* kernels = kF64 ? fp64 : P->form == kSmall ? small : P->form == kMid ? mid : wide;
-    for (int k = 0; k < 4 && kernels[k]; ++k)
-        if (cudaFuncSetAttribute(kernels[k], cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max - 512) != cudaSuccess)
-            return true;
-    int per_sm = 0;
-    const void* all = kF64 ? kernels[0] : kernels[3];
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, all, kF64 ? kThreads64 : P->threads_a, P->smem_a) != cudaSuccess) return true;
-    P->one_launch = ctrl && m <= per_sm * sms && m <= kOneLaunchRows;
     P->fp64 = kF64;
-    if (kF64 && !P->one_launch) return false;
+    // the same limit for every plan: a function's attribute is shared by all of them
+    auto allow = [&](const void* k) {
+        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max - 512) == cudaSuccess;
+    };
+    int per_sm = 0;
+    const void* all = kF64 ? (const void*)k_dst_fp64 : (const void*)kernel_all(*P);
+    if (!allow(all) ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, all, kF64 ? kThreads64 : P->threads_a, P->smem_a) != cudaSuccess)
+        return true;
+    P->one_launch = m <= per_sm * sms && m <= kOneLaunchRows;
+    if (!P->one_launch) {
+        // (a device with room for fewer blocks than a GB300; there the small forms always fit)
+        if (kF64 || P->form == kSmall || (P->form == kMid && F.cols_b == 1)) return false;
+        if (!allow((const void*)kernel_a(*P)) || !allow((const void*)kernel_b(*P)) || !allow((const void*)kernel_c(*P))) return true;
+    }
     // copies from pageable memory may still be on their way, and the callers' streams do not wait for the default one
     if (cudaDeviceSynchronize() != cudaSuccess) return true;
     *status = CNV_OK;
@@ -1252,18 +1250,19 @@ int dst_plan_create(int n, int Lx, int Ly, Ctrl* ctrl, long long timeout_ns, int
     int status = CNV_OK;
     const DstPlan bare = *P;
     if (m <= kFp64Rows && fp64_radix_ok(m + 1)) {
-        if (plan_fft<double>(P, Ly / g, Lx / g, sms, smem_max, ctrl, &status)) {
+        if (plan_fft<double>(P, Ly / g, Lx / g, sms, smem_max, &status)) {
             if (status != CNV_OK) dst_plan_destroy(P);
             return status;
         }
         dst_plan_destroy(P);
         *P = bare;
     }
-    if (plan_fft<float>(P, Ly / g, Lx / g, sms, smem_max, ctrl, &status)) {
+    if (plan_fft<float>(P, Ly / g, Lx / g, sms, smem_max, &status)) {
         if (status != CNV_OK) dst_plan_destroy(P);
         return status;
     }
-    P->F = FftArgs{};
+    dst_plan_destroy(P);
+    *P = bare;
     // dense products with the DST matrix
     const double pi = std::acos(-1.0);
     std::vector<double> S((size_t)m * m);

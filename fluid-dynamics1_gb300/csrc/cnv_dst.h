@@ -67,7 +67,7 @@ struct DstPlan {
     void* arena = nullptr;     // the FFT path's tables and fields
 };
 
-// Lx and Ly are the cavity's extents (dx = Lx / n, dy = Ly / n). ctrl (may be null) takes the status and the abort flag
+// Lx and Ly are the cavity's extents (dx = Lx / n, dy = Ly / n). ctrl takes the status and the abort flag
 // of a solve whose blocks wait for one another (bounded by timeout_ns). stall_block: see DstPlan (-1: none).
 int dst_plan_create(int n, int Lx, int Ly, Ctrl* ctrl, long long timeout_ns, int stall_block, DstPlan* plan);
 // Re-arm the barrier after a solve that timed out: once before the solves of a call.
