@@ -121,6 +121,7 @@ struct cnv_state {
     void* msync = nullptr;
     int mixed_gx = 1, mixed_gy = 1, mixed_epochs = 1, mixed_max_outer = 100;
     bool mixed_rq_smem = false;
+    size_t mixed_smem_max = 0;
     int mixed_form = -1, mixed_ntx = 0, mixed_nty = 0;
     double mixed_rtol = 1e-10;
     // several sweeps per border exchange (FP64 SOR/GS in shared-memory tiles)
@@ -311,6 +312,7 @@ MixedLaunch mixed_launch(cnv_state* s) {
     L.max_outer = s->mixed_max_outer;
     L.epochs = s->mixed_epochs;
     L.rq_in_smem = s->mixed_rq_smem ? 1 : 0;
+    L.smem_max = s->mixed_smem_max;
     L.form = s->mixed_form;
     L.ntx = s->mixed_ntx;
     L.nty = s->mixed_nty;
@@ -564,9 +566,10 @@ int cnv_create(const cnv_config* cfg, cnv_state** out) {
             for (g = std::min(s->sms, kMaxSolverBlocks); g >= 1 && !tiles_ok(g);) --g;
             if (g < 1) s->mixed_gx = s->mixed_gy = 1;
         }
-        s->mixed_rq_smem = mixed_smem_bytes(n, s->mixed_gx, s->mixed_gy, true) + 2048 <= prop.sharedMemPerBlockOptin;
+        s->mixed_smem_max = prop.sharedMemPerBlockOptin - 2048;
+        s->mixed_rq_smem = mixed_smem_bytes(n, s->mixed_gx, s->mixed_gy, true) <= s->mixed_smem_max;
         const size_t smem = mixed_smem_bytes(n, s->mixed_gx, s->mixed_gy, s->mixed_rq_smem);
-        if (smem + 2048 > prop.sharedMemPerBlockOptin) {
+        if (smem > s->mixed_smem_max) {
             free_state(s);
             return fail(CNV_BAD_ARG, "grid %d too large for the mixed form (tile needs %zu B of shared memory)", n,
                         smem);

@@ -81,6 +81,7 @@ struct MixedLaunch {
     int max_outer, epochs;
     int form, ntx, nty;  // register kernel's form and threads across and down its box (form -1: shared-memory tiles)
     int rq_in_smem;   // keep the correction right-hand side tile in shared memory
+    size_t smem_max;  // dynamic shared memory that any solve may ask for
     long long timeout_ns;
     int stall_block;  // testing only: block that never publishes its border (-1: none)
     const double* g[2];

@@ -865,7 +865,8 @@ cudaError_t launch_mixed(const MixedLaunch& L, cudaStream_t s) {
         smem = (size_t)kForms[L.form].units(threads) * 16;
         kernel = kForms[L.form].kernel;
     }
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // one limit for all solves: the attribute belongs to the function, and another thread may launch it between the two calls
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem_max);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(L.gx * L.gy);
