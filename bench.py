@@ -545,9 +545,9 @@ def ours(args):
     fp64 = None
     add_mul, fma_rate = cnvpy.probe_fp64(local)
     if args.form == "fp64":
-        # the binding ceiling: the update's 7 FP64 add/multiply operations per interior cell-sweep
-        # (5 on the FP64 pipe, the 2 multiplications by constants in exact integer arithmetic),
-        # against the device's own FP64 rate for that mix (probe kernels, same process)
+        # for comparison (the FP64 and the integer pipe take turns, neither binds alone): the update's
+        # 7 FP64 add/multiply operations per interior cell-sweep (5 on the FP64 pipe, the 2
+        # multiplications by constants in exact integer arithmetic), against the device's own FP64 rate for that mix (probe kernels, same process)
         ops = 7.0 * interior * sweeps / (pms * 1e-3)
         fp64 = {"achieved_gops": round(ops / 1e9, 1), "peak_gops": round(add_mul / 1e9, 1),
                 "frac": round(ops / add_mul, 4), "fma_peak_gops": round(fma_rate / 1e9, 1),

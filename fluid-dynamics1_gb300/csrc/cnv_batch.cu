@@ -824,7 +824,8 @@ int group_size(int n, int smem_bytes, int split, int min_n) {
 // shared memory, 1.5 k from L2), with the halo rows of a strip, plus the FP64 passes; and for a
 // group, its barriers: one per 4 FP32 sweeps (the border-row swap) plus about 20 around the
 // residual norms and the passes, each about kBarrierUs (the wait for the slowest strip and the
-// halo rows' L2 round trip), which the strips cannot share out.
+// halo rows' L2 round trip), which the strips cannot share out. The rates are those of the scalar sweeps; the vector sweeps do
+// about 9 k cells/us, so the estimates are too high (256 cavities 35.3 ms, measured 18.7; ten of 192^2 3.72 and 2.79).
 constexpr double kBarrierUs = 3.5;
 
 double step_cost(int n, int g, int smem_mode) {

@@ -248,7 +248,8 @@ int cnv_batch_groups(cnv_batch *b, int *groups);
 /* Host only, no device needed: the row strips per cavity (groups, count entries) that
  * cnv_batch_create picks on a device that runs `blocks` batch blocks of `smem_bytes` bytes of
  * shared memory each (a GB300: 152 and 231424), and the schedule's estimated step time in
- * microseconds (makespan_us, may be NULL). */
+ * microseconds (makespan_us, may be NULL; made with the rates of scalar sweeps, so up to twice
+ * the measured time where the correction is in shared memory). */
 int cnv_batch_plan(int count, const cnv_cavity_spec *specs, int blocks, int smem_bytes, int *groups,
                    double *makespan_us);
 /* Advance every cavity nsteps steps in one launch; last (count records or NULL) receives each
